@@ -70,9 +70,23 @@ struct gf2c_decoder {
   int lay_stage_off = 0, lay_stage_bytes = 0;
   const void* kernel = nullptr;
   bool state_flood = false;  // check-state flooding min-sum kernel (state_flood.cu)
-  int sf_app_soff = 0;
+  int sf_app_soff = 0, sf_tab_off = -1;
+  // check-state kernel, frame state on chip: CTAs of 1024, 512 and 256 threads
+  // in flight (0: not used); a launch takes the smallest CTA whose slots its
+  // frames still fill, so that the SMs hold as many warps as they can
+  int sf_slots[3] = {0, 0, 0};
+  // the kernel with the frame state in the workspace, for clusters of 2, 4, 8
+  // and 16 CTAs per frame (clusters in flight; 0: not used): a batch that leaves
+  // SMs idle takes the largest team that decodes it in one wave.  50 iterations
+  // of one normal 3/5 frame: 5.36 ms by one CTA, 2.88 / 1.57 / 0.94 / 0.61 ms by
+  // teams of 2 / 4 / 8 / 16; short 1/2: 0.95 ms, 0.70 / 0.51 / 0.40 / 0.33 ms.
+  // For a full batch one CTA per frame stays ahead (normal 3/5, 1000 frames:
+  // 32.3 ms, teams of 2: 32.7 ms).
+  const void* sf_team_kernel = nullptr;
+  StateFloodLayout sf_team{};
+  int sf_teams[5] = {0, 0, 0, 0, 0};
   long long sf_llr_off = 0, sf_st_off = 0, sf_app_off = 0;
-  size_t smem = 0;
+  size_t smem = 0, work_bytes = 0;
   long long work_stride = 0, app_offset = 0;
   DevBuf work, queue, status, alpha, beta;
   int nms_iters = 0, nms_L = 0;
@@ -302,6 +316,22 @@ int gf2c_channel_awgn(const gf2c_code* code, uint64_t seed, uint64_t frame0, int
 // ---------------------------------------------------------------------------
 static const int kSmemBudget = 200 * 1024;
 
+// Launch configuration of a check-state decode by teams of `size` CTAs.
+static cudaLaunchConfig_t team_config(const gf2c_decoder* d, int size, int teams, cudaStream_t st,
+                                      cudaLaunchAttribute* at) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)size;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)(size * teams));
+  c.blockDim = dim3((unsigned)state_flood_threads());
+  c.dynamicSmemBytes = d->sf_team.smem;
+  c.stream = st;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return c;
+}
+
 int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, const gf2c_decoder_opts* opts,
                               gf2c_decoder** out) {
   if (!out || !codes || ncodes <= 0) return set_error(GF2C_ERR_INVALID_ARG, "bad arguments");
@@ -456,26 +486,17 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   const int sf_dc = state_dcmax_bucket(d->max_dc);
   if (!layered && ms_family && sf_dc > 0 && !std::getenv("GF2C_NO_STATE_FLOOD") &&
       (o.threads_per_block == 0 || o.threads_per_block == state_flood_threads())) {
-    const size_t budget = 224 * 1024;
-    const size_t st_bytes = (size_t)d->max_m * 16, app_bytes = (size_t)d->max_n * 4;
-    bool any_perm = false;
-    for (auto* c : d->codes) any_perm = any_perm || !c->h->sp_u2v.empty();
-    // Either the whole frame state is on chip, or all of it is in the workspace:
-    // keeping only part of it in shared memory (measured on normal 3/5 frames)
-    // shrinks L1, which caches the workspace, by more than it saves in L2 traffic.
-    const bool all_smem = st_bytes + app_bytes <= budget;
-    d->sf_app_soff = (int)st_bytes;
-    auto al = [](long long x) { return (x + 255) / 256 * 256; };
-    long long off = 0;
-    d->sf_llr_off = off;
-    off += any_perm ? al(app_bytes) : 0;
-    d->sf_st_off = off;
-    off += all_smem ? 0 : al(st_bytes);
-    d->sf_app_off = off;
-    off += all_smem ? 0 : al(app_bytes);
-    d->work_stride = off;
-    d->smem = all_smem ? st_bytes + app_bytes : 0;
-    d->kernel = state_flood_kernel_ptr(sf_dc, all_smem);
+    std::vector<const HostCode*> hc;
+    for (auto* c : d->codes) hc.push_back(c->h.get());
+    const StateFloodLayout L = state_flood_layout(hc);
+    d->sf_app_soff = L.app_soff;
+    d->sf_tab_off = L.tab_off;
+    d->sf_llr_off = L.llr_off;
+    d->sf_st_off = L.st_off;
+    d->sf_app_off = L.app_off;
+    d->work_stride = L.work_stride;
+    d->smem = L.smem;
+    d->kernel = state_flood_kernel_ptr(sf_dc, L.all_smem);
     d->dcmax = sf_dc;
     threads = state_flood_threads();
     d->threads = threads;
@@ -550,7 +571,44 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   if (occ <= 0) return set_error(GF2C_ERR_UNSUPPORTED, "decode kernel does not fit on an SM with this shape");
   int bps = o.blocks_per_sm ? std::min(o.blocks_per_sm, occ) : occ;
   d->grid = sms * bps;
-  if ((rc = d->work.ensure((size_t)d->work_stride * d->grid))) return rc;
+  if (d->state_flood && d->sf_tab_off >= 0 && d->sf_st_off == d->sf_app_off && o.threads_per_block == 0 &&
+      o.blocks_per_sm == 0) {
+    // Small codes leave most of a 1024-thread CTA's warps waiting at the two
+    // barriers of an iteration; smaller CTAs put several frames on an SM.
+    for (int i = 0; i < 3; i++) {
+      int b = 0;
+      GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, d->kernel, threads >> i, d->smem));
+      d->sf_slots[i] = sms * b;
+      d->grid = std::max(d->grid, d->sf_slots[i]);
+    }
+  }
+  size_t work_bytes = (size_t)d->work_stride * d->grid;
+  // A team's barriers cost about 5 us per iteration, one CTA about 0.4 ns per
+  // edge: a small code (a 2304-bit code of 8 K edges: 0.16 ms by one CTA, 0.20 ms
+  // by two) stays with one.
+  int64_t min_edges = INT64_MAX;
+  for (auto* c : d->codes) min_edges = std::min(min_edges, (int64_t)c->h->row_idx.size());
+  if (d->state_flood && o.threads_per_block == 0 && o.blocks_per_sm == 0 && min_edges >= 24000) {
+    std::vector<const HostCode*> hc;
+    for (auto* c : d->codes) hc.push_back(c->h.get());
+    d->sf_team = state_flood_layout(hc, false);
+    d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, false);
+    GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->sf_team.smem));
+    GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int lg = 1; lg <= 4; lg++) {
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = team_config(d.get(), 1 << lg, 1, nullptr, &at);
+      int nc = 0;
+      if (cudaOccupancyMaxActiveClusters(&nc, d->sf_team_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        nc = 0;
+      }
+      d->sf_teams[lg] = nc;
+      work_bytes = std::max(work_bytes, (size_t)d->sf_team.work_stride * nc);
+    }
+  }
+  if ((rc = d->work.ensure(work_bytes))) return rc;
+  d->work_bytes = work_bytes;
   if ((rc = d->queue.ensure(64)) || (rc = d->status.ensure(64))) return rc;
   GF2C_CUDA(cudaMemset(d->status.p, 0, 64));
   *out = d.release();
@@ -598,15 +656,40 @@ static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaSt
   a.early_stop = d->opts.early_stop;
   a.status = (int*)d->status.p;
   a.sf_app_soff = d->sf_app_soff;
+  a.sf_tab_off = d->sf_tab_off;
   a.sf_msg16 = d->opts.msg_dtype == GF2C_MSG_F16;
   a.sf_llr_off = d->sf_llr_off;
   a.sf_st_off = d->sf_st_off;
   a.sf_app_off = d->sf_app_off;
   GF2C_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), st));
-  int grid = (int)std::min<int64_t>(d->grid, frames);
+  int team = 0;
+  for (int lg = 4; lg >= 1 && !team; lg--)
+    if (frames <= d->sf_teams[lg]) team = lg;
+  if (team) {
+    a.work_stride = d->sf_team.work_stride;
+    a.sf_app_soff = d->sf_team.app_soff;
+    a.sf_tab_off = d->sf_team.tab_off;
+    a.sf_llr_off = d->sf_team.llr_off;
+    a.sf_st_off = d->sf_team.st_off;
+    a.sf_app_off = d->sf_team.app_off;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg =
+        team_config(d, 1 << team, (int)std::min<int64_t>(d->sf_teams[team], frames), st, &at);
+    d->last_launches = 1;
+    void* args[] = {(void*)&a};
+    GF2C_CUDA(cudaLaunchKernelExC(&cfg, d->sf_team_kernel, args));
+    return GF2C_OK;
+  }
+  int grid = (int)std::min<int64_t>(d->grid, frames), threads = d->threads;
+  if (d->sf_slots[0] > 0) {
+    int i = 0;
+    while (i < 2 && frames >= d->sf_slots[i + 1] && d->sf_slots[i + 1] > d->sf_slots[i]) i++;
+    threads >>= i;
+    grid = (int)std::min<int64_t>(d->sf_slots[i], frames);
+  }
   d->last_launches = 1;
   void* args[] = {(void*)&a};
-  GF2C_CUDA(cudaLaunchKernel(d->kernel, dim3(grid), dim3(d->threads), args, d->smem, st));
+  GF2C_CUDA(cudaLaunchKernel(d->kernel, dim3(grid), dim3(threads), args, d->smem, st));
   return GF2C_OK;
 }
 
@@ -680,7 +763,7 @@ static bool pipeline_ready(gf2c_decoder* d) {
       cudaGetLastError();
       return false;
     }
-  if (d->work2.ensure((size_t)d->work_stride * d->grid) != GF2C_OK || d->queue2.ensure(64) != GF2C_OK) {
+  if (d->work2.ensure(d->work_bytes) != GF2C_OK || d->queue2.ensure(64) != GF2C_OK) {
     cudaGetLastError();  // an allocation failure: the call runs unpipelined
     return false;
   }

@@ -142,6 +142,78 @@ static bool finish_plan(HostCode& c) {
   return true;
 }
 
+// Structured variable edge lists of a code whose check slots all fit the
+// descriptors (see DevCode::sp_mode); checked entry by entry against the edge
+// table, which stays in use when any variable does not match.
+static void plan_structured(HostCode& c) {
+  c.sp_mode = 0;
+  c.sp_vh.clear();
+  c.sp_vd.clear();
+  c.sp_rot.clear();
+  const int Z = c.z;
+  if (c.sp_desc.empty() || Z <= 0 || c.vgs != Z || c.n % Z != 0 || c.m * 16 >= (1ll << 31)) return;
+  for (size_t g = 0; g < c.cg.size(); g++) {
+    const uint32_t ab = c.sp_absent[g];
+    const int d = c.cg[g].z;
+    // the one slot without an edge: the staircase corner (first check, last slot but one)
+    if (c.cg[g].y != Z || c.cg[g].x != (int)g * Z || (ab && !(g == 0 && d >= 2 && ab == 1u << (d - 2)))) return;
+  }
+  const int nvg = (int)(c.n / Z);
+  struct Circ {
+    int g, slot, tau;
+  };
+  std::vector<std::vector<Circ>> of(nvg);
+  for (size_t g = 0; g < c.sp_cg.size(); g++)
+    for (int i = 0; i < c.sp_cg[g].z; i++) {
+      const int2 D = c.sp_desc[(size_t)c.sp_cg[g].w + i];
+      const int base = D.x - (Z - D.y);  // first variable of the circulant's block
+      if (base % Z != 0) return;
+      of[base / Z].push_back(Circ{(int)g, i, D.y % Z});
+    }
+  const bool rot = c.kind == 2;
+  if (rot) c.sp_rot.assign((size_t)c.n, 0);
+  for (int h = 0; h < nvg; h++) {
+    auto& L = of[h];
+    const int dv = (int)L.size();
+    if (rot)
+      std::sort(L.begin(), L.end(), [](const Circ& x, const Circ& y) { return x.tau != y.tau ? x.tau < y.tau : x.g < y.g; });
+    if (dv > 63) return;
+    c.sp_vh.push_back(int2{dv, (int)c.sp_vd.size()});
+    if (rot) {
+      for (int pass = 0; pass < 2; pass++)
+        for (const Circ& e : L) c.sp_vd.push_back(int2{16 * (e.g * Z + e.tau - (pass == 0 ? Z : 0)), e.slot});
+    } else {
+      for (const Circ& e : L) c.sp_vd.push_back(int2{16 * (e.g * Z + e.tau), e.slot | (Z - e.tau) << 8});
+    }
+    for (int j = 0; j < Z; j++) {
+      int s = 0, cnt = dv;
+      if (rot) {
+        s = dv;  // the first circulant that wraps
+        for (int i = dv - 1; i >= 0 && j + L[i].tau >= Z; i--) s = i;
+        // the staircase corner: its wrapped entry has no edge (it is the first of the list)
+        if (s < dv && L[s].g == 0 && c.sp_absent[0] == 1u << L[s].slot && j + L[s].tau == Z) {
+          s++;
+          cnt--;
+        }
+        c.sp_rot[(size_t)h * Z + j] = (uint8_t)(s | (cnt < dv ? 128 : 0));
+      }
+      const int2 V = c.sp_vg[h];
+      for (int i = 0; i < V.x; i++) {
+        const int want = c.sp_ci[(size_t)V.y + (size_t)i * Z + j];
+        int have = -1;
+        if (i < cnt) {
+          const int2 e = c.sp_vd[(size_t)c.sp_vh[h].y + s + i];
+          const int wrap = rot ? Z : e.y >> 8;
+          have = (e.x / 16 + j - (j >= wrap ? Z : 0)) | (e.y & 0xff) << 24;
+        }
+        if (have != want) return;
+      }
+      if (cnt > V.x) return;
+    }
+  }
+  c.sp_mode = rot ? 1 : 2;
+}
+
 // Check-state flooding plan.  DVB-T2 parity bits are stored transposed (u order,
 // see DevCode); every other code keeps the natural order.  For codes with slot
 // descriptors each (CG, slot) is refitted in u order as base + (t + shift) mod Z
@@ -237,6 +309,7 @@ void plan_state(HostCode& c) {
     for (int j0 = 0; j0 < vgs && (int64_t)h * vgs + j0 < n; j0 += 32) c.sp_vchunk.push_back(int2{h, j0});
   }
   c.sp_vg = vg2;
+  plan_structured(c);
 }
 
 // Generic plan: CGs of up to 256 consecutive checks, slots in CSR order.
@@ -587,6 +660,12 @@ int upload_code(HostCode& c) {
     if ((rc = dev_copy(c, c.sp_u2v, &d.sp_u2v))) return rc;
     d.sp_ncchunk = (int)c.sp_cchunk.size();
     d.sp_nvchunk = (int)c.sp_vchunk.size();
+    d.sp_mode = c.sp_mode;
+    d.sp_nvd = (int)c.sp_vd.size();
+    d.sp_ndesc = (int)c.sp_desc.size();
+    if ((rc = dev_copy(c, c.sp_vh, &d.sp_vh))) return rc;
+    if ((rc = dev_copy(c, c.sp_vd, &d.sp_vd))) return rc;
+    if ((rc = dev_copy(c, c.sp_rot, &d.sp_rot))) return rc;
     std::vector<int> rp(c.row_ptr.begin(), c.row_ptr.end()), ri(c.row_idx.begin(), c.row_idx.end());
     if ((rc = dev_copy(c, rp, &d.csr_ptr))) return rc;
     if ((rc = dev_copy(c, ri, &d.csr_idx))) return rc;

@@ -68,6 +68,21 @@ struct DevCode {
   const int2* sp_vchunk;           // var chunks {var group, first j}: 32 variables of one group
   int sp_nvchunk;
   const int* sp_u2v;               // natural index of u-order variable u (nullptr: identity)
+  // Structured variable edge lists (QC / DVB-T2 codes; sp_mode 0: none, use
+  // sp_ci).  Edge lists per var group, {16 * (state index offset), slot |
+  // wrap << 8}: the state of entry e for variable j of the group is at byte
+  // offset e.x + 16 j, minus 16 Z when j >= wrap (sp_mode 2, QC codes: a fixed
+  // edge order).  sp_mode 1 (DVB-T2): ascending original check index is
+  // ascending position t = (j + tau) mod Z, i.e. the circulants sorted by tau
+  // and rotated so that the wrapped ones come first; the list holds the
+  // wrapped and then the unwrapped circulants, and variable u starts at entry
+  // sp_rot[u] & 127 (bit 7: one edge fewer, the staircase's last variable).
+  int sp_mode;
+  const int2* sp_vh;               // per var group {edges, first list entry}
+  const int2* sp_vd;
+  const uint8_t* sp_rot;
+  int sp_nvd;                      // list entries of all groups
+  int sp_ndesc;                    // entries of sp_desc
   const int* csr_ptr;              // natural order H (m + 1)
   const int* csr_idx;              // (nnz)
   // encoder
@@ -114,6 +129,9 @@ struct HostCode {
   std::vector<uint32_t> sp_absent;
   std::vector<int2> sp_cchunk, sp_vchunk, sp_vg;
   std::vector<int> sp_ci, sp_u2v;
+  int sp_mode = 0;
+  std::vector<int2> sp_vh, sp_vd;
+  std::vector<uint8_t> sp_rot;
 
   // encoder (generic)
   int enc_kind = 0;
@@ -203,6 +221,7 @@ struct DecodeArgs {
   // LLRs, the check states and the posteriors (frame state in the workspace)
   int sf_msg16;
   int sf_app_soff;
+  int sf_tab_off;                  // byte offset in shared memory of the structured tables (-1: not used)
   long long sf_llr_off, sf_st_off, sf_app_off;
 };
 
@@ -221,6 +240,16 @@ cudaError_t launch_failed_list(const uint8_t* syndrome_ok, int64_t frames, int64
                                cudaStream_t st);
 int state_dcmax_bucket(int max_dc);
 int state_flood_threads();
+// Memory layout of the check-state kernel for a set of codes: frame state in
+// shared memory (all_smem) or in the CTA's workspace slice, then the tables of
+// the structured passes in shared memory (tab_off -1: no structured pass).
+struct StateFloodLayout {
+  bool all_smem;
+  size_t smem;
+  int app_soff, tab_off;
+  long long llr_off, st_off, app_off, work_stride;
+};
+StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, bool on_chip = true);
 const void* state_flood_kernel_ptr(int dcmax, bool all_smem);
 int decode_dcmax_bucket(int max_dc);
 int layered_dcmax_bucket(int max_dc);

@@ -89,7 +89,7 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
     size_t off;
   };
   // the generic flooding kernel's tables, then the check-state kernel's
-  Part parts[14] = {{h.cg.data(), h.cg.size() * sizeof(int4), 0},
+  Part parts[17] = {{h.cg.data(), h.cg.size() * sizeof(int4), 0},
                     {h.chk_cg.data(), h.chk_cg.size() * sizeof(uint16_t), 0},
                     {h.slot_var.data(), h.slot_var.size() * sizeof(int), 0},
                     {h.slot_desc.data(), h.slot_desc.size() * sizeof(uint32_t), 0},
@@ -102,7 +102,10 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
                     {h.sp_vg.data(), h.sp_vg.size() * sizeof(int2), 0},
                     {h.sp_ci.data(), h.sp_ci.size() * sizeof(int), 0},
                     {h.sp_vchunk.data(), h.sp_vchunk.size() * sizeof(int2), 0},
-                    {h.sp_u2v.data(), h.sp_u2v.size() * sizeof(int), 0}};
+                    {h.sp_u2v.data(), h.sp_u2v.size() * sizeof(int), 0},
+                    {h.sp_vh.data(), h.sp_vh.size() * sizeof(int2), 0},
+                    {h.sp_vd.data(), h.sp_vd.size() * sizeof(int2), 0},
+                    {h.sp_rot.data(), h.sp_rot.size() * sizeof(uint8_t), 0}};
   for (auto& pt : parts) {
     pt.off = off;
     off = align256(off + pt.bytes);
@@ -117,21 +120,18 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
   const int bitmap_words = (int)((h.n + 31) / 32);
   const size_t kSmemBudget = 200 * 1024;
   const void* kern = nullptr;
-  int threads = 512, smem_app = 0;
+  int threads = 512, smem_app = 0, sf_tab_off = -1;
   size_t smem = 0, work_stride = 0, c2v_bytes = 0, st_bytes = 0, sf_llr_off = 0, sf_st_off = 0, sf_app_off = 0;
   if (state) {
-    st_bytes = (size_t)h.m * 16;
-    const size_t app_bytes = (size_t)h.n * 4;
-    const bool all_smem = st_bytes + app_bytes <= 224 * 1024;
-    size_t o = 0;
-    sf_llr_off = o;
-    o += h.sp_u2v.empty() ? 0 : align256(app_bytes);
-    sf_st_off = o;
-    o += all_smem ? 0 : align256(st_bytes);
-    sf_app_off = o;
-    o += all_smem ? 0 : align256(app_bytes);
-    work_stride = o;
-    smem = all_smem ? st_bytes + app_bytes : 0;
+    const StateFloodLayout L = state_flood_layout({&h});
+    sf_llr_off = L.llr_off;
+    sf_st_off = L.st_off;
+    sf_app_off = L.app_off;
+    work_stride = L.work_stride;
+    smem = L.smem;
+    sf_tab_off = L.tab_off;
+    st_bytes = L.app_soff;
+    const bool all_smem = L.all_smem;
     kern = state_flood_kernel_ptr(sf_dc, all_smem);
     threads = state_flood_threads();
   } else {
@@ -184,6 +184,12 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
     d.sp_vchunk = (const int2*)at(12);
     d.sp_nvchunk = (int)h.sp_vchunk.size();
     d.sp_u2v = (const int*)at(13);
+    d.sp_mode = h.sp_mode;
+    d.sp_vh = (const int2*)at(14);
+    d.sp_vd = (const int2*)at(15);
+    d.sp_rot = (const uint8_t*)at(16);
+    d.sp_nvd = (int)h.sp_vd.size();
+    d.sp_ndesc = (int)h.sp_desc.size();
     for (auto& pt : parts)
       if (pt.bytes) GF2C_CUDA(cudaMemcpyAsync(S.base + pt.off, pt.src, pt.bytes, cudaMemcpyHostToDevice, st));
     S.dev = d;
@@ -231,6 +237,7 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
   a.early_stop = 1;
   a.sf_msg16 = 0;
   a.sf_app_soff = (int)st_bytes;
+  a.sf_tab_off = sf_tab_off;
   a.sf_llr_off = (long long)sf_llr_off;
   a.sf_st_off = (long long)sf_st_off;
   a.sf_app_off = (long long)sf_app_off;
