@@ -67,8 +67,14 @@ struct gf2c_decoder {
   int max_n = 0, max_m = 0, max_words_k = 0, max_e_slots = 0, max_dc = 0, max_nchk = 0;
   int dcmax = 0, threads = 0, grid = 0, bitmap_words = 0, smem_app_floats = 0;
   int lay_dbuf_off = 0, lay_dbuf_floats = 0;
-  int lay_stage_off = 0, lay_stage_bytes = 0;
+  int lay_stage_off = 0, lay_stage_bytes = 0, lay_tab_off = 0;
   const void* kernel = nullptr;
+  // Layered min-sum family on normal DVB-T2 frames with FP16 messages, for more
+  // frames than `grid` holds: two checks per thread, four frames per SM (8192
+  // normal 2/3 frames: 26.1 ms against 28.9 ms; the sum-product, whose rows hold
+  // more registers, and short frames lose: 2048 normal 3/5 frames 59 -> 72 ms).
+  const void* lay_many_kernel = nullptr;
+  int lay_many_threads = 0, lay_many_grid = 0, lay_few_grid = 0;
   bool state_flood = false;  // check-state flooding min-sum kernel (state_flood.cu)
   int sf_app_soff = 0, sf_tab_off = -1;
   // check-state kernel, frame state on chip: CTAs of 1024, 512 and 256 threads
@@ -467,18 +473,43 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   d->work_stride = c2v_bytes + (need_gapp ? ((long long)d->max_n * 4 + 255) / 256 * 256 : 0);
   d->kernel = layered ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads)
                       : flood_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads);
-  if (layered && threads <= 384) {
-    // codes of different slot counts (a mixed batch): the kernel that runs each
-    // frame with its own code's exact slot count, where one exists
-    bool differ = false, dispatchable = true;
+  if (multi_mixed && d->dcmax <= 22) d->kernel = layered_kernel_ptr(o.algorithm, o.msg_dtype, 0, threads);
+  // DVB-T2 codes with a fused-row algorithm: their own kernels, one code or a
+  // mixed batch.  Shared memory: bitmap, posteriors (short frames), the deltas
+  // of the slots inside runs of one block, the tables.
+  bool dvb = false;
+  if (layered && o.algorithm != GF2C_ALGO_SPA && threads <= 384) {
+    const bool mixed = d->codes.size() > 1;
+    int D = mixed ? 0 : layered_dvb_bucket(*d->codes[0]->h), runs = 0;
+    size_t tab = 0;
+    bool all = true;
     for (auto* c : d->codes) {
-      const int b = layered_dcmax_bucket(c->h->max_dc);
-      differ = differ || b != d->dcmax;
-      dispatchable = dispatchable && b > 0 && b <= 22;
+      const HostCode& h = *c->h;
+      all = all && layered_dvb_bucket(h) > 0;
+      for (uint32_t s : h.cg_sync) runs = std::max(runs, __builtin_popcount(s | s << 1));
+      tab = std::max(tab, h.cg.size() * 16 + h.sp_desc.size() * 8);
     }
-    const void* k = ((differ || multi_mixed) && dispatchable) ? layered_kernel_ptr(o.algorithm, o.msg_dtype, 0, threads)
-                                                               : nullptr;
-    if (k) d->kernel = k;
+    const bool shared_app = d->smem_app_floats > 0;
+    const void* k = all ? layered_dvb_kernel_ptr(o.algorithm, o.msg_dtype, D, shared_app, threads) : nullptr;
+    if (k) {
+      dvb = true;
+      d->kernel = k;
+      size_t off = (smem_of(d->smem_app_floats) + 15) & ~(size_t)15;
+      d->lay_dbuf_off = (int)off;
+      d->lay_dbuf_floats = runs * d->max_nchk;
+      off += (size_t)d->lay_dbuf_floats * 4;
+      d->lay_tab_off = (int)off;
+      d->smem = off + tab;
+      if (!shared_app && o.algorithm != GF2C_ALGO_SPA_FAST && msg_bytes == 2 && o.threads_per_block == 0 &&
+          o.blocks_per_sm == 0) {
+        d->lay_many_threads = 192;
+        d->lay_many_kernel = layered_dvb_kernel_ptr(o.algorithm, o.msg_dtype, D, false, 192);
+      }
+      if (o.algorithm != GF2C_ALGO_SPA_FAST) {  // compressed states only
+        d->app_offset = ((long long)d->max_m * (o.msg_dtype == GF2C_MSG_F16 ? 8 : 16) + 255) / 256 * 256;
+        d->work_stride = d->app_offset + (need_gapp ? ((long long)d->max_n * 4 + 255) / 256 * 256 : 0);
+      }
+    }
   }
   // Flooding min-sum / normalised-offset min-sum: the check-state kernel, with
   // the check states and posteriors in shared memory where they fit.
@@ -506,7 +537,9 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     return set_error(GF2C_ERR_INVALID_ARG,
                      "flooding schedule: threads_per_block above 512 needs a code of check degree <= 8");
   if (!d->kernel && !multi) return set_error(GF2C_ERR_UNSUPPORTED, "no decode kernel for this configuration");
-  if (multi && d->lay_dbuf_floats > 0) {
+  if (dvb) {
+    // laid out above
+  } else if (multi && d->lay_dbuf_floats > 0) {
     // several checks per thread: the delta buffer is required
     d->smem = (size_t)d->lay_dbuf_off + (size_t)d->lay_dbuf_floats * 4;
   } else if (d->lay_dbuf_floats > 0) {
@@ -529,7 +562,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   // of each row group are staged in shared memory by TMA bulk copies (a row
   // group's messages are one contiguous block, which must start and end on a
   // 16-byte boundary; three or more row groups), where this costs no occupancy.
-  if (layered && d->codes.size() == 1 && o.algorithm != GF2C_ALGO_SPA && threads <= 384 &&
+  if (layered && !dvb && d->codes.size() == 1 && o.algorithm != GF2C_ALGO_SPA && threads <= 384 &&
       !std::getenv("GF2C_NO_STAGE")) {
     const HostCode& h = *d->codes[0]->h;
     // the min-sum family keeps compressed check states and stages nothing (the
@@ -542,7 +575,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
       ok = ok && (states || (off % 16 == 0 && by % 16 == 0));
       if (!states) mx = std::max(mx, by);
     }
-    const void* k = ok ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads, true, o.blocks_per_sm)
+    const void* k = ok ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads, true)
                        : nullptr;
     int optin = 0, occ0 = 0, occ1 = 0;
     GF2C_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->dev));
@@ -581,6 +614,14 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
       d->sf_slots[i] = sms * b;
       d->grid = std::max(d->grid, d->sf_slots[i]);
     }
+  }
+  d->lay_few_grid = d->grid;
+  if (d->lay_many_kernel) {
+    int b = 0;
+    GF2C_CUDA(cudaFuncSetAttribute(d->lay_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
+    GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, d->lay_many_kernel, d->lay_many_threads, d->smem));
+    d->lay_many_grid = sms * b;
+    d->grid = std::max(d->grid, d->lay_many_grid);
   }
   size_t work_bytes = (size_t)d->work_stride * d->grid;
   // A team's barriers cost about 5 us per iteration, one CTA about 0.4 ns per
@@ -644,6 +685,7 @@ static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaSt
   a.bitmap_words = d->bitmap_words;
   a.lay_dbuf_off = d->lay_dbuf_off;
   a.lay_dbuf_floats = d->lay_dbuf_floats;
+  a.lay_tab_off = d->lay_tab_off;
   a.lay_stage_off = d->lay_stage_off;
   a.lay_stage_bytes = d->lay_stage_bytes;
   a.alpha = (const float*)d->alpha.p;
@@ -687,9 +729,18 @@ static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaSt
     threads >>= i;
     grid = (int)std::min<int64_t>(d->sf_slots[i], frames);
   }
+  const void* kernel = d->kernel;
+  if (d->lay_many_kernel) {
+    const bool many = frames > d->lay_few_grid;
+    if (many) {
+      kernel = d->lay_many_kernel;
+      threads = d->lay_many_threads;
+    }
+    grid = (int)std::min<int64_t>(many ? d->lay_many_grid : d->lay_few_grid, frames);
+  }
   d->last_launches = 1;
   void* args[] = {(void*)&a};
-  GF2C_CUDA(cudaLaunchKernel(d->kernel, dim3(grid), dim3(threads), args, d->smem, st));
+  GF2C_CUDA(cudaLaunchKernel(kernel, dim3(grid), dim3(threads), args, d->smem, st));
   return GF2C_OK;
 }
 

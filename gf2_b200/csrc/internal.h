@@ -208,6 +208,7 @@ struct DecodeArgs {
   int smem_app_floats;             // APP kept in shared memory when n <= this
   int bitmap_words;                // 32-bit words of the hard-decision bitmap
   int lay_dbuf_off, lay_dbuf_floats;  // layered fused rows: shared-memory buffer of slots x checks
+  int lay_tab_off;                    // DVB-T2 layered kernels: row-group records and slot descriptors in smem
   int lay_stage_off, lay_stage_bytes; // layered, TMA-staged messages: two buffers of one row group's
                                       // messages, then two mbarriers (byte offset in dynamic smem)
   const float* alpha;              // NMS weights [nms_iters][nms_L]
@@ -253,8 +254,12 @@ StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, b
 const void* state_flood_kernel_ptr(int dcmax, bool all_smem);
 int decode_dcmax_bucket(int max_dc);
 int layered_dcmax_bucket(int max_dc);
-// bps: requested CTAs per SM (0 = any); 192 threads with 5 or more picks the 64-register build
-const void* layered_kernel_ptr(int algo, int msg16, int dcmax, int maxt, bool stage = false, int bps = 0);
+const void* layered_kernel_ptr(int algo, int msg16, int dcmax, int maxt, bool stage = false);
+// DVB-T2 layered kernels (layered_dvb.cuh): slot bucket of a code they decode
+// (0: none), and the kernel for bucket D (0: a mixed batch), the posteriors'
+// placement and 384, 192 or 128 threads (nullptr: none).
+int layered_dvb_bucket(const HostCode& h);
+const void* layered_dvb_kernel_ptr(int algo, int msg16, int D, bool shared_app, int threads);
 size_t layered_smem_bytes(int smem_app_floats, int bitmap_words);
 // Layered min-sum / normalised-offset min-sum on the single-code (staged)
 // kernels with the fused row paths: one compressed state per check (8 bytes
