@@ -638,6 +638,8 @@ int upload_code(HostCode& c) {
     d.layered_ok = c.layered_ok;
     d.lay_bucket = layered_dcmax_bucket(c.max_dc);
     d.max_nchk = c.max_nchk;
+    d.lay_dvb = layered_dvb_bucket(c);
+    for (uint32_t x : c.cg_sync) d.lay_runs = std::max(d.lay_runs, __builtin_popcount(x | x << 1));
     int rc;
     if ((rc = dev_copy(c, c.cg, &d.cg))) return rc;
     if ((rc = dev_copy(c, c.cg_sync, &d.cg_sync))) return rc;

@@ -35,6 +35,8 @@ struct DevCode {
   int layered_ok;                  // CGs are layers usable by the layered schedule
   int lay_bucket;                  // slot count of the layered kernel that fits this code exactly
   int max_nchk;                    // largest CG
+  int lay_dvb;                     // DVB-T2 layered kernels: slot bucket (0: not one of their codes)
+  int lay_runs;                    // most slots inside runs of one block in a row group
   const int4* cg;                  // {chk_begin, nchk, dc, edge0}
   const uint32_t* cg_sync;         // layered: bit i = barrier after slot i (dup variables)
   const int* slot_var;             // [e_slots]
@@ -281,6 +283,9 @@ int launch_nms_layered(const DevCode* dcode, const DevCode& h, int T, int L, con
                        long long frames, const float* alpha, const float* beta, float* X, float* B, char* work,
                        long long work_stride, int grid, float* pf, float* ga, float* gb, float* loss,
                        cudaStream_t st);
+int launch_nms_layered_dvb(const DevCode* dcode, const DevCode& h, int T, int L, const float* llr, const uint64_t* cw,
+                           long long frames, const float* alpha, const float* beta, float* X, float* B, char* work,
+                           long long work_stride, int grid, float* pf, cudaStream_t st);
 int launch_count_errors(const uint64_t* a, const uint64_t* b, long long frames, int words, int32_t* per_frame,
                         unsigned long long* totals, cudaStream_t st);
 int launch_adam(float* p, const float* g, float* m1, float* m2, int count, float lr, float b1, float b2, float eps,

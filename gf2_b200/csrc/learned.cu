@@ -551,13 +551,19 @@ int launch_nms_layered(const DevCode* dcode, const DevCode& h, int T, int L, con
   if (h.max_dc > kLearnDcMax) return set_error(GF2C_ERR_UNSUPPORTED, "learned decoder: check degree above 32");
   if (!h.layered_ok || h.max_nchk > kLayThreadsMax)
     return set_error(GF2C_ERR_UNSUPPORTED, "layered training needs row groups of at most 1024 checks");
-  const int threads = std::max(32, (h.max_nchk + 31) / 32 * 32);
-  nms_layered_forward_kernel<<<grid, threads, 0, st>>>(dcode, T, L, llr, cw, frames, alpha, beta, X, B, work,
-                                                        work_stride, pf);
-  GF2C_CUDA(cudaGetLastError());
-  nms_layered_backward_kernel<<<grid, threads, 0, st>>>(dcode, T, L, cw, frames, alpha, beta, X, B, work,
-                                                         work_stride, pf);
-  GF2C_CUDA(cudaGetLastError());
+  if (h.lay_dvb) {
+    const int rc = launch_nms_layered_dvb(dcode, h, T, L, llr, cw, frames, alpha, beta, X, B, work, work_stride, grid,
+                                          pf, st);
+    if (rc) return rc;
+  } else {
+    const int threads = std::max(32, (h.max_nchk + 31) / 32 * 32);
+    nms_layered_forward_kernel<<<grid, threads, 0, st>>>(dcode, T, L, llr, cw, frames, alpha, beta, X, B, work,
+                                                          work_stride, pf);
+    GF2C_CUDA(cudaGetLastError());
+    nms_layered_backward_kernel<<<grid, threads, 0, st>>>(dcode, T, L, cw, frames, alpha, beta, X, B, work,
+                                                           work_stride, pf);
+    GF2C_CUDA(cudaGetLastError());
+  }
   const int outs = 2 * T * L + 1, warps = 8;
   nms_reduce_kernel<<<(outs + warps - 1) / warps, warps * 32, 0, st>>>(pf, frames, T * L, ga, gb, loss);
   GF2C_CUDA(cudaGetLastError());
