@@ -78,7 +78,7 @@ class BchEncoder:
         if hasattr(msg_words, "data_ptr"):
             import torch
             F = msg_words.shape[0]
-            out = torch.zeros((F, words(c.n())), dtype=torch.int64, device=msg_words.device)
+            out = torch.empty((F, words(c.n())), dtype=torch.int64, device=msg_words.device)
             st = stream or torch.cuda.current_stream(msg_words.device)
             C.check(C.lib.gf2c_bch_encode_batch(c.handle, _ptr(msg_words.contiguous()), F, _ptr(out), C.MEM_DEVICE,
                                                 _stream_ptr(st)))
@@ -111,10 +111,10 @@ class BchDecoder:
             import torch
             F = cw_words.shape[0]
             dev = cw_words.device
-            out = dict(msg=torch.zeros((F, words(c.k())), dtype=torch.int64, device=dev),
-                       corrected=torch.zeros(F, dtype=torch.int32, device=dev))
+            out = dict(msg=torch.empty((F, words(c.k())), dtype=torch.int64, device=dev),
+                       corrected=torch.empty(F, dtype=torch.int32, device=dev))
             if syndromes:
-                out["syndromes"] = torch.zeros((F, 2 * c.t()), dtype=torch.int16, device=dev)
+                out["syndromes"] = torch.empty((F, 2 * c.t()), dtype=torch.int16, device=dev)
             st = stream or torch.cuda.current_stream(dev)
             C.check(C.lib.gf2c_bch_decode_batch(c.handle, _ptr(cw_words.contiguous()), F, _ptr(out["msg"]),
                                                 _ptr(out["corrected"]), _ptr(out.get("syndromes")), C.MEM_DEVICE,

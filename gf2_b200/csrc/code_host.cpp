@@ -674,6 +674,7 @@ int upload_code(HostCode& c) {
     d.enc_kind = c.kind == 2 ? 0 : 1;
     if (c.kind == 2) {
       d.enc_q = c.q;
+      d.enc_rg_total = (int)c.enc_rg_ent.size();
       if ((rc = dev_copy(c, c.enc_rg_ptr, &d.enc_rg_ptr))) return rc;
       if ((rc = dev_copy(c, c.enc_rg_ent, &d.enc_rg_ent))) return rc;
     }

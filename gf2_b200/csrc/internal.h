@@ -93,6 +93,7 @@ struct DevCode {
   const int* enc_msg_cols;         // kind 1: k message columns
   const int* enc_par_cols;         // kind 1: m parity columns
   int enc_q;                       // kind 0: row groups (m / 360)
+  int enc_rg_total;                // kind 0: entries of enc_rg_ent
   const int* enc_rg_ptr;           // kind 0: q + 1 offsets into enc_rg_ent
   const int* enc_rg_ent;           // kind 0: info block b << 16 | rotation tau, per row group
 };

@@ -325,8 +325,8 @@ class LdpcCode:
         if hasattr(cw_bits_packed, "data_ptr"):
             import torch
             F = cw_bits_packed.shape[0]
-            s = torch.zeros((F, words(self._m)), dtype=torch.int64, device=cw_bits_packed.device)
-            w = torch.zeros(F, dtype=torch.int32, device=cw_bits_packed.device)
+            s = torch.empty((F, words(self._m)), dtype=torch.int64, device=cw_bits_packed.device)
+            w = torch.empty(F, dtype=torch.int32, device=cw_bits_packed.device)
             C.check(C.lib.gf2c_syndrome_batch(self._h, _ptr(cw_bits_packed), F, _ptr(s), _ptr(w), C.MEM_DEVICE,
                                               _stream_ptr(stream or torch.cuda.current_stream())))
             return s, w
@@ -474,12 +474,12 @@ class LdpcDecoder:
         F = llr.shape[0]
         dev = llr.device
         if out is None:
-            out = dict(msg=torch.zeros((F, words(self.k())), dtype=torch.int64, device=dev),
-                       iters=torch.zeros(F, dtype=torch.int32, device=dev),
-                       conv=torch.zeros(F, dtype=torch.uint8, device=dev),
-                       synd_ok=torch.zeros(F, dtype=torch.uint8, device=dev))
+            out = dict(msg=torch.empty((F, words(self.k())), dtype=torch.int64, device=dev),
+                       iters=torch.empty(F, dtype=torch.int32, device=dev),
+                       conv=torch.empty(F, dtype=torch.uint8, device=dev),
+                       synd_ok=torch.empty(F, dtype=torch.uint8, device=dev))
             if beliefs:
-                out["beliefs"] = torch.zeros((F, self.n()), dtype=torch.float32, device=dev)
+                out["beliefs"] = torch.empty((F, self.n()), dtype=torch.float32, device=dev)
         st = stream or torch.cuda.current_stream(dev)
         C.check(C.lib.gf2c_decode_batch(self._h, _ptr(llr), F, int(max_iterations), _ptr(out["msg"]),
                                         _ptr(out["iters"]), _ptr(out["conv"]), _ptr(out["synd_ok"]),
@@ -529,10 +529,10 @@ class LdpcDecoder:
                 out = {k: (v.numpy() if hasattr(v, "numpy") else v) for k, v in out.items()}
             return out
         if out is None:
-            out = dict(msg=torch.zeros((F, words(self.k())), dtype=torch.int64, device=dev),
-                       iters=torch.zeros(F, dtype=torch.int32, device=dev),
-                       conv=torch.zeros(F, dtype=torch.uint8, device=dev),
-                       synd_ok=torch.zeros(F, dtype=torch.uint8, device=dev),
+            out = dict(msg=torch.empty((F, words(self.k())), dtype=torch.int64, device=dev),
+                       iters=torch.empty(F, dtype=torch.int32, device=dev),
+                       conv=torch.empty(F, dtype=torch.uint8, device=dev),
+                       synd_ok=torch.empty(F, dtype=torch.uint8, device=dev),
                        fallback_count=torch.zeros(1, dtype=torch.int64, device=dev))
         st = stream or torch.cuda.current_stream(dev)
         C.check(C.lib.gf2c_decode_batch_fallback(self._h, fallback._h, _ptr(llr), F, int(max_iterations),
@@ -608,7 +608,7 @@ class LdpcEncoder:
         if hasattr(msg_packed, "data_ptr"):
             import torch
             F = msg_packed.shape[0]
-            cw = torch.zeros((F, words(self.n())), dtype=torch.int64, device=msg_packed.device)
+            cw = torch.empty((F, words(self.n())), dtype=torch.int64, device=msg_packed.device)
             C.check(C.lib.gf2c_encode_batch(self.code.handle, _ptr(msg_packed), F, _ptr(cw), C.MEM_DEVICE,
                                             _stream_ptr(stream or torch.cuda.current_stream())))
             return cw
@@ -653,8 +653,8 @@ def awgn_frames(code, seed, frame0, frames, sigma2, device=None, want_info=True,
         return info, cw, llr
     import torch
     s2 = torch.as_tensor(np.broadcast_to(np.asarray(sigma2, np.float64), (frames,)).copy(), device=device)
-    info = torch.zeros((frames, words(code.k())), dtype=torch.int64, device=device) if want_info else None
-    cw = torch.zeros((frames, words(code.n())), dtype=torch.int64, device=device) if want_cw else None
+    info = torch.empty((frames, words(code.k())), dtype=torch.int64, device=device) if want_info else None
+    cw = torch.empty((frames, words(code.n())), dtype=torch.int64, device=device) if want_cw else None
     llr = torch.empty((frames, code.n()), dtype=torch.float32, device=device)
     C.check(C.lib.gf2c_channel_awgn(code.handle, int(seed), int(frame0), int(frames), _ptr(s2), _ptr(info),
                                     _ptr(cw), _ptr(llr), C.MEM_DEVICE,
