@@ -91,6 +91,8 @@ struct gf2c_decoder {
   const void* sf_team_kernel = nullptr;
   StateFloodLayout sf_team{};
   int sf_teams[5] = {0, 0, 0, 0, 0};
+  int team_threads = 0;
+  bool spa_flood = false;  // flooding sum-product of one DVB-T2 code (spa_flood.cu)
   long long sf_llr_off = 0, sf_st_off = 0, sf_app_off = 0;
   size_t smem = 0, work_bytes = 0;
   long long work_stride = 0, app_offset = 0;
@@ -330,7 +332,7 @@ static cudaLaunchConfig_t team_config(const gf2c_decoder* d, int size, int teams
   at->val.clusterDim.y = at->val.clusterDim.z = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = dim3((unsigned)(size * teams));
-  c.blockDim = dim3((unsigned)state_flood_threads());
+  c.blockDim = dim3((unsigned)d->team_threads);
   c.dynamicSmemBytes = d->sf_team.smem;
   c.stream = st;
   c.attrs = at;
@@ -533,6 +535,21 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     d->threads = threads;
     d->state_flood = true;
   }
+  if (!layered && !ms_family && o.threads_per_block == 0 && o.blocks_per_sm == 0 && d->codes.size() == 1 &&
+      layered_dvb_bucket(*d->codes[0]->h) > 0) {
+    const void* k = spa_flood_kernel_ptr(o.algorithm, o.msg_dtype, layered_dvb_bucket(*d->codes[0]->h));
+    if (k) {
+      d->kernel = d->sf_team_kernel = k;
+      d->sf_team = spa_flood_layout({d->codes[0]->h.get()}, (int)msg_bytes);
+      d->work_stride = d->sf_team.work_stride;
+      d->sf_llr_off = d->sf_team.llr_off;
+      d->sf_st_off = d->sf_team.st_off;
+      d->sf_app_off = d->sf_team.app_off;
+      d->smem = d->sf_team.smem;
+      threads = d->threads = d->team_threads = spa_flood_threads();
+      d->spa_flood = true;
+    }
+  }
   if (!layered && !d->state_flood && threads > 512 && !d->kernel)
     return set_error(GF2C_ERR_INVALID_ARG,
                      "flooding schedule: threads_per_block above 512 needs a code of check degree <= 8");
@@ -629,11 +646,15 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   // by two) stays with one.
   int64_t min_edges = INT64_MAX;
   for (auto* c : d->codes) min_edges = std::min(min_edges, (int64_t)c->h->row_idx.size());
-  if (d->state_flood && o.threads_per_block == 0 && o.blocks_per_sm == 0 && min_edges >= 24000) {
-    std::vector<const HostCode*> hc;
-    for (auto* c : d->codes) hc.push_back(c->h.get());
-    d->sf_team = state_flood_layout(hc, false);
-    d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, false);
+  if (d->spa_flood ||
+      (d->state_flood && o.threads_per_block == 0 && o.blocks_per_sm == 0 && min_edges >= 24000)) {
+    if (d->state_flood) {
+      std::vector<const HostCode*> hc;
+      for (auto* c : d->codes) hc.push_back(c->h.get());
+      d->sf_team = state_flood_layout(hc, false);
+      d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, false);
+      d->team_threads = state_flood_threads();
+    }
     GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->sf_team.smem));
     GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     for (int lg = 1; lg <= 4; lg++) {
@@ -672,6 +693,39 @@ int gf2c_decoder_last_launches(const gf2c_decoder* dec, int32_t* launches) {
   return GF2C_OK;
 }
 
+// CTAs per frame (log2) of a flooding decode of `frames` frames.  Min-sum: the
+// team with the shortest estimate, waves times the time of a frame (relative to
+// one CTA, measured on short 1/2 with its state on chip and on normal 3/5:
+// sf_teams).  Sum-product: frames differ more in iterations than in anything
+// else, so a few waves of larger teams beat one of smaller ones (37 short 1/2
+// frames: 0.87 ms by teams of 4, 0.74 ms by teams of 8 in three waves), and two
+// CTAs per frame beat one for every batch (1000 frames 8.4 ms both, 256 frames
+// 2.69 against 3.27 ms, 2.78 ms by teams of 4).
+static int team_of(const gf2c_decoder* d, int64_t frames) {
+  if (d->spa_flood) {
+    if (frames <= d->sf_teams[4]) return 4;
+    if (frames <= 3 * (int64_t)d->sf_teams[3]) return 3;
+    if (frames <= 3 * (int64_t)d->sf_teams[2]) return 2;
+    return d->sf_teams[1] > 0 ? 1 : 0;
+  }
+  if (!d->sf_team_kernel) return 0;
+  static const float on_chip[5] = {1.0f, 0.74f, 0.54f, 0.42f, 0.35f};
+  static const float in_memory[5] = {1.0f, 0.54f, 0.29f, 0.175f, 0.113f};
+  const float* t = d->sf_st_off == d->sf_app_off ? on_chip : in_memory;
+  int best = 0;
+  float cost = 0.0f;
+  for (int lg = 0; lg <= 4; lg++) {
+    const int64_t slots = lg ? d->sf_teams[lg] : std::max(d->sf_slots[0], d->grid);
+    if (slots <= 0) continue;
+    const float c = (float)((frames + slots - 1) / slots) * t[lg];
+    if (lg == 0 || c < cost) {
+      best = lg;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 // slot 1: the second workspace and queue of the pipelined host-memory path
 static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaStream_t st, int slot = 0) {
   a.codes = (const DevCode*)d->d_codes.p;
@@ -704,9 +758,7 @@ static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaSt
   a.sf_st_off = d->sf_st_off;
   a.sf_app_off = d->sf_app_off;
   GF2C_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), st));
-  int team = 0;
-  for (int lg = 4; lg >= 1 && !team; lg--)
-    if (frames <= d->sf_teams[lg]) team = lg;
+  const int team = team_of(d, frames);
   if (team) {
     a.work_stride = d->sf_team.work_stride;
     a.sf_app_soff = d->sf_team.app_soff;
@@ -752,7 +804,8 @@ static int launch_decoder(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaSt
 // number of kernels launched (0 or 2) in `launches`.
 static int key_order(gf2c_decoder* d, DecodeArgs& a, int64_t frames, cudaStream_t st, int slot, int& launches) {
   launches = 0;
-  if (d->codes.size() != 1 || frames <= d->grid || frames > kKeyOrderMax) return GF2C_OK;
+  const int team = team_of(d, frames);
+  if (d->codes.size() != 1 || frames <= (team ? d->sf_teams[team] : d->grid) || frames > kKeyOrderMax) return GF2C_OK;
   DevBuf& kb = d->d_key[slot];
   DevBuf& ob = d->d_korder[slot];
   if (kb.bytes < (size_t)frames * 4 || ob.bytes < (size_t)frames * 8) {

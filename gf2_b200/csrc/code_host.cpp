@@ -150,6 +150,7 @@ static void plan_structured(HostCode& c) {
   c.sp_vh.clear();
   c.sp_vd.clear();
   c.sp_rot.clear();
+  c.sp_ve.clear();
   const int Z = c.z;
   if (c.sp_desc.empty() || Z <= 0 || c.vgs != Z || c.n % Z != 0 || c.m * 16 >= (1ll << 31)) return;
   for (size_t g = 0; g < c.cg.size(); g++) {
@@ -181,7 +182,11 @@ static void plan_structured(HostCode& c) {
     c.sp_vh.push_back(int2{dv, (int)c.sp_vd.size()});
     if (rot) {
       for (int pass = 0; pass < 2; pass++)
-        for (const Circ& e : L) c.sp_vd.push_back(int2{16 * (e.g * Z + e.tau - (pass == 0 ? Z : 0)), e.slot});
+        for (const Circ& e : L) {
+          const int t0 = e.tau - (pass == 0 ? Z : 0);
+          c.sp_vd.push_back(int2{16 * (e.g * Z + t0), e.slot});
+          c.sp_ve.push_back(c.cg[e.g].w + e.slot * Z + t0 - h * Z);
+        }
     } else {
       for (const Circ& e : L) c.sp_vd.push_back(int2{16 * (e.g * Z + e.tau), e.slot | (Z - e.tau) << 8});
     }
@@ -668,6 +673,7 @@ int upload_code(HostCode& c) {
     if ((rc = dev_copy(c, c.sp_vh, &d.sp_vh))) return rc;
     if ((rc = dev_copy(c, c.sp_vd, &d.sp_vd))) return rc;
     if ((rc = dev_copy(c, c.sp_rot, &d.sp_rot))) return rc;
+    if ((rc = dev_copy(c, c.sp_ve, &d.sp_ve))) return rc;
     std::vector<int> rp(c.row_ptr.begin(), c.row_ptr.end()), ri(c.row_idx.begin(), c.row_idx.end());
     if ((rc = dev_copy(c, rp, &d.csr_ptr))) return rc;
     if ((rc = dev_copy(c, ri, &d.csr_idx))) return rc;

@@ -83,6 +83,8 @@ struct DevCode {
   const int2* sp_vh;               // per var group {edges, first list entry}
   const int2* sp_vd;
   const uint8_t* sp_rot;
+  const int* sp_ve;                // sp_mode 1: per list entry the message index of (row group, slot) plus
+                                   // the position offset, minus the var group's first variable
   int sp_nvd;                      // list entries of all groups
   int sp_ndesc;                    // entries of sp_desc
   const int* csr_ptr;              // natural order H (m + 1)
@@ -135,6 +137,7 @@ struct HostCode {
   int sp_mode = 0;
   std::vector<int2> sp_vh, sp_vd;
   std::vector<uint8_t> sp_rot;
+  std::vector<int> sp_ve;
 
   // encoder (generic)
   int enc_kind = 0;
@@ -255,6 +258,10 @@ struct StateFloodLayout {
 };
 StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, bool on_chip = true);
 const void* state_flood_kernel_ptr(int dcmax, bool all_smem);
+// Flooding sum-product on DVB-T2 codes (spa_flood.cu), one kernel per bucket D of slots.
+int spa_flood_threads();
+StateFloodLayout spa_flood_layout(const std::vector<const HostCode*>& codes, int msg_bytes);
+const void* spa_flood_kernel_ptr(int algo, int msg16, int D);
 int decode_dcmax_bucket(int max_dc);
 int layered_dcmax_bucket(int max_dc);
 const void* layered_kernel_ptr(int algo, int msg16, int dcmax, int maxt, bool stage = false);

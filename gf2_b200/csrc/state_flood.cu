@@ -46,7 +46,7 @@
 
 #include <algorithm>
 
-#include "internal.h"
+#include "flood_common.cuh"
 #include "numeric.cuh"
 
 namespace gf2c {
@@ -69,38 +69,6 @@ struct Post {
   float* p;
   __device__ __forceinline__ float* at(int u) const { return p + u; }
   __device__ __forceinline__ float* run(int) const { return p; }
-};
-
-// A frame may be decoded by a cluster of CTAs (frame state in the workspace,
-// shared by the cluster): warps of all its CTAs take the chunks, and the frame's
-// barriers are cluster barriers, whose release / acquire makes one CTA's writes
-// visible to the others.
-struct Team {
-  int size, rank;     // CTAs, this CTA
-  int warp, nwarps;   // this warp among all warps of the team
-  __device__ __forceinline__ void sync() const {
-    if (size == 1) {
-      __syncthreads();
-    } else {
-      asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
-    }
-  }
-  // Stores v to the shared variable at p in every CTA of the team.
-  __device__ __forceinline__ void put(int* p, int v) const {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    for (int r = 0; r < size; r++)
-      asm volatile("{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %0, %1;\n st.shared::cluster.u32 [ra], %2;\n}" ::"r"(a),
-                   "r"(r), "r"(v)
-                   : "memory");
-  }
-  // Barrier that returns whether any thread of the team passes p != 0; flag is
-  // zero when the first thread arrives (every CTA has its own copy).
-  __device__ __forceinline__ int any(int p, int* flag) const {
-    if (size == 1) return __syncthreads_or(p);
-    if (__any_sync(0xffffffffu, p) && (threadIdx.x & 31) == 0) put(flag, 1);
-    sync();
-    return *(volatile int*)flag;
-  }
 };
 
 struct SlotTables {
@@ -193,28 +161,10 @@ __device__ __forceinline__ int check_node(const float (&ap)[DCMAX], uint32_t rea
 // 37.5 -> 31.7 ms by loading the next variables' LLRs ahead, taking two
 // degree-3 variables at a time and reading the LLRs evict-first).
 // ---------------------------------------------------------------------------
-struct FastTab {
-  const int2* desc;  // slot descriptors {start, wrap}
-  const int2* cg;    // per row group {slots, first descriptor}
-  const int2* vh;    // per var group {edges, first list entry}
-  const int2* vd;    // edge lists
-};
-
 // Check-node update of check t of a row group whose D slots all hold an edge.
 // `corner` (the staircase's first check): the slot before the last holds none
 // and reads the +inf posterior at index n, which leaves minima and signs as
 // they are.  Returns a word whose bit 31 is the parity of the hard decisions.
-template <int D>
-__device__ __forceinline__ void load_check(const int2* sd, int t, int Z, const float* P, bool corner, int n,
-                                           float (&ap)[D]) {
-#pragma unroll
-  for (int i = 0; i < D; i++) {
-    const int2 S = sd[i];
-    int u = S.x + t - (t >= S.y ? Z : 0);
-    if (i == D - 2) u = corner ? n : u;
-    ap[i] = P[u];
-  }
-}
 template <int D>
 __device__ __forceinline__ uint32_t update_check(const float (&ap)[D], const uint4 so, uint4* st_cc, bool nms, float al,
                                                  float be, bool msg16) {
@@ -517,13 +467,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
   __shared__ int s_frame[2];  // the frame (low, high word)
   __shared__ int s_vote[3];   // team votes: alternating iterations, final syndrome
   const DevCode& C = sf_code;
-  Team team{1, 0, 0, 0};
-  if (!ALL_SMEM) {
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(team.size));
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(team.rank));
-  }
-  team.warp = team.rank * ((int)blockDim.x >> 5) + ((int)threadIdx.x >> 5);
-  team.nwarps = team.size * ((int)blockDim.x >> 5);
+  const Team team = Team::make(!ALL_SMEM);
   // thread index and count of the team
   const int tid = team.rank * (int)blockDim.x + (int)threadIdx.x, NT = team.size * (int)blockDim.x;
   const int lane = threadIdx.x & 31, ltid = threadIdx.x, LT = blockDim.x;
@@ -595,16 +539,8 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
     const bool fast = a.sf_tab_off >= 0 && C.sp_mode != 0;
     FastTab T{};
     if (fast) {
-      int2* tab = (int2*)(smem_raw + a.sf_tab_off);
-      const int nd = C.sp_ndesc, ncg = C.ncg, nvg = C.n / C.vgs, nvd = C.sp_nvd;
-      T = FastTab{tab, tab + nd, tab + nd + ncg, tab + nd + ncg + nvg};
-      if (tab_code != cid) {
-        for (int i = ltid; i < nd; i += LT) tab[i] = __ldg(&C.sp_desc[i]);
-        for (int i = ltid; i < ncg; i += LT) tab[nd + i] = make_int2(__ldg(&C.sp_cg[i]).z, __ldg(&C.sp_cg[i]).w);
-        for (int i = ltid; i < nvg; i += LT) tab[nd + ncg + i] = __ldg(&C.sp_vh[i]);
-        for (int i = ltid; i < nvd; i += LT) tab[nd + ncg + nvg + i] = __ldg(&C.sp_vd[i]);
-        tab_code = cid;
-      }
+      T = stage_tables(C, (int2*)(smem_raw + a.sf_tab_off), tab_code != cid);
+      tab_code = cid;
       if (tid == 0) P.p[n] = __int_as_float(0x7f800000);  // what the staircase corner reads
     }
     const float* lu = u2v ? llr_u : llr;
