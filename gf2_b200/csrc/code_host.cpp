@@ -432,10 +432,15 @@ int build_dvbt2(int frame, int rate, HostCode& c) {
   c.m = m;
   c.n = n;
   std::vector<std::vector<int64_t>> per_row(m);
+  for (auto& row : per_row) row.reserve(24);
   for (int b = 0; b < T.rows; b++)
     for (int a = T.row_ptr[b]; a < T.row_ptr[b + 1]; a++) {
       int64_t x = T.addr[a];
-      for (int64_t j = 0; j < Z; j++) per_row[(x + j * q) % m].push_back(b * Z + j);
+      for (int64_t j = 0; j < Z; j++) {
+        per_row[x].push_back(b * Z + j);
+        x += q;
+        if (x >= m) x -= m;
+      }
     }
   for (int64_t p = 0; p < m; p++) {
     per_row[p].push_back(k + p);
