@@ -315,6 +315,12 @@ void plan_state(HostCode& c) {
   }
   c.sp_vg = vg2;
   plan_structured(c);
+  if (!c.sp_mode) {
+    c.sp_vh.clear();
+    c.sp_vd.clear();
+    c.sp_rot.clear();
+    c.sp_ve.clear();
+  }
 }
 
 // Generic plan: CGs of up to 256 consecutive checks, slots in CSR order.

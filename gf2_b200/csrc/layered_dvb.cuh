@@ -438,8 +438,8 @@ __device__ __forceinline__ void dvb_iterations(const DecodeArgs& a, const DevCod
 // batch, normal 5/6: 16.7 against 3.3 ms).  Not staged in shared memory by TMA:
 // the stage's L1 and proxy fences cost what it hid (2048 normal 3/5 frames 59.0
 // against 57.7 ms, short 3/4 5.2 against 4.5 ms).  8192 normal 2/3 frames,
-// min-sum: 43.5 -> 26.1 ms; 2048 normal 3/5, sum-product: 82.4 -> 57.7 ms;
-// 4096 short 3/4, sum-product: 7.3 -> 4.5 ms.  Three CTAs of 384 threads per SM
+// min-sum: 43.5 -> 26.1 ms; 2048 normal 3/5, sum-product: 82.4 -> 57.7 ms (56.5
+// with the L2 prefetch); 4096 short 3/4, sum-product: 7.3 -> 4.5 ms.  Three CTAs of 384 threads per SM
 // (56 registers) spill: 57.7 -> 84 ms.  D = 0: a mixed batch, each frame with
 // its own code's slot count (PL then is where short frames live, normal ones
 // are in the workspace).

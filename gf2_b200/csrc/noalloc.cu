@@ -88,7 +88,12 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
     size_t bytes;
     size_t off;
   };
-  // the generic flooding kernel's tables, then the check-state kernel's
+  // the check-state kernel where it covers the code, else the generic one
+  const int sf_dc = state_dcmax_bucket(h.max_dc);
+  const bool state = sf_dc > 0 && !std::getenv("GF2C_NO_STATE_FLOOD");
+  const StateFloodLayout L = state ? state_flood_layout({&h}) : StateFloodLayout{};
+  // the generic flooding kernel's tables, then the check-state kernel's; those of
+  // its structured passes only where the kernel runs them
   Part parts[17] = {{h.cg.data(), h.cg.size() * sizeof(int4), 0},
                     {h.chk_cg.data(), h.chk_cg.size() * sizeof(uint16_t), 0},
                     {h.slot_var.data(), h.slot_var.size() * sizeof(int), 0},
@@ -106,24 +111,21 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
                     {h.sp_vh.data(), h.sp_vh.size() * sizeof(int2), 0},
                     {h.sp_vd.data(), h.sp_vd.size() * sizeof(int2), 0},
                     {h.sp_rot.data(), h.sp_rot.size() * sizeof(uint8_t), 0}};
+  if (!state || L.tab_off < 0) parts[14].bytes = parts[15].bytes = parts[16].bytes = 0;
   for (auto& pt : parts) {
     pt.off = off;
     off = align256(off + pt.bytes);
   }
   const size_t tables_end = off;
 
-  // kernel and per-CTA workspace: the check-state kernel where it covers the
-  // code (frame state on chip when it fits, else in the workspace), else the
-  // generic flooding kernel with FP32 messages
-  const int sf_dc = state_dcmax_bucket(h.max_dc);
-  const bool state = sf_dc > 0 && !std::getenv("GF2C_NO_STATE_FLOOD");
+  // kernel and per-CTA workspace: check-state kernel with the frame state on chip
+  // when it fits, else in the workspace; generic kernel with FP32 messages
   const int bitmap_words = (int)((h.n + 31) / 32);
   const size_t kSmemBudget = 200 * 1024;
   const void* kern = nullptr;
   int threads = 512, smem_app = 0, sf_tab_off = -1;
   size_t smem = 0, work_stride = 0, c2v_bytes = 0, st_bytes = 0, sf_llr_off = 0, sf_st_off = 0, sf_app_off = 0;
   if (state) {
-    const StateFloodLayout L = state_flood_layout({&h});
     sf_llr_off = L.llr_off;
     sf_st_off = L.st_off;
     sf_app_off = L.app_off;

@@ -636,11 +636,13 @@ StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, b
   // shrinks L1, which caches the workspace, by more than it saves in L2 traffic.
   // The tables go beside it up to the most a CTA may have (1 KB left for the
   // static part), and up to 48 KB, so that most of L1 stays a cache.
-  const size_t st_bytes = max_m * 16, app_bytes = (max_n * 4 + 4 + 15) / 16 * 16;  // one more posterior: the corner's
+  const size_t st_bytes = max_m * 16;
   StateFloodLayout L{};
   L.all_smem = on_chip && st_bytes + max_n * 4 <= 224 * 1024;
+  size_t app_bytes = (max_n * 4 + 4 + 15) / 16 * 16;  // one more posterior: the corner's
   const size_t state = L.all_smem ? st_bytes + app_bytes : 0;
   const bool fits = any_fast && tab <= 48 * 1024 && state + tab <= 226 * 1024;
+  if (!fits) app_bytes = max_n * 4;
   L.app_soff = (int)st_bytes;
   L.tab_off = fits ? (int)state : -1;
   L.smem = fits ? state + tab : (L.all_smem ? st_bytes + max_n * 4 : 0);

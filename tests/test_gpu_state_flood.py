@@ -78,3 +78,30 @@ def test_structured_flooding_nms_fp16_equals_oracle(gpu, oracle, frames):
     assert (r["iters"] == o["iters"][0]).all() and (r["conv"] == o["conv"][0]).all()
     assert (g.unpack_bits(r["msg"], code.k()) == o["msg"]).all()
     assert np.array_equal(r["beliefs"], np.repeat(o["beliefs"], frames, 0), equal_nan=True)
+
+
+def test_noalloc_takes_a_code_just_inside_its_scratch(gpu):
+    """A QC code whose structured tables (43 KB and more) are too large for shared
+    memory and would exceed the 64 MiB scratch, of which the rest of it leaves 30 KB:
+    it is decoded without them, bit for bit like the allocating entry point."""
+    import ctypes
+
+    import torch
+    from gf2_b200 import _capi as C
+    mb, nb, Z, dc = 500, 1000, 914, 10
+    base = np.full((mb, nb), -1, np.int32)
+    for r in range(mb):
+        for i in range(dc):
+            c = r if i == 0 else mb + r if i == 1 else (r * 5 + i * 3) % nb
+            base[r, c] = (r * 37 + c * 11) % Z
+    code = g.LdpcCode._create(C.lib.gf2c_code_create_qc, base.ctypes.data_as(ctypes.c_void_p), mb, nb, Z)
+    gen = torch.Generator(device=gpu).manual_seed(3)
+    llr = torch.randn((1, code.n()), generator=gen, device=gpu) + 1.0
+    ref = g.LdpcDecoder(code).decode_tensors(llr, 2)
+    msg = torch.zeros((1, g.words(code.k())), dtype=torch.int64, device=gpu)
+    it = torch.zeros(1, dtype=torch.int32, device=gpu)
+    cv, so = (torch.zeros(1, dtype=torch.uint8, device=gpu) for _ in range(2))
+    C.check(C.lib.gf2c_decode_batch_noalloc(code.handle, ctypes.c_void_p(llr.data_ptr()), 1, 2,
+                                            *(ctypes.c_void_p(t.data_ptr()) for t in (msg, it, cv, so)), None))
+    torch.cuda.synchronize()
+    assert torch.equal(msg, ref["msg"]) and torch.equal(it, ref["iters"]) and torch.equal(cv, ref["conv"])
