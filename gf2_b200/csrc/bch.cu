@@ -824,15 +824,33 @@ struct gf2c_bch {
 
 namespace {
 
-template <class T>
-int dev_upload(gf2c_bch* b, const std::vector<T>& v, const T** out) {
-  void* p = nullptr;
-  GF2C_CUDA(cudaMalloc(&p, std::max(sizeof(T) * v.size(), (size_t)16)));
-  b->allocs.push_back(p);
-  GF2C_CUDA(cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
-  *out = (const T*)p;
-  return GF2C_OK;
-}
+// The code's tables in one device allocation, 256-byte aligned parts.
+struct BchUpload {
+  struct Part {
+    const void* src;
+    size_t bytes;
+    const void** out;
+  };
+  std::vector<Part> parts;
+  template <class T, class U>
+  void add(const std::vector<T>& v, const U** out) {
+    parts.push_back(Part{v.data(), sizeof(T) * v.size(), (const void**)out});
+  }
+  int run(gf2c_bch* b) {
+    auto padded = [](size_t x) { return (x + 255) / 256 * 256; };
+    size_t total = 256;
+    for (const Part& p : parts) total += padded(p.bytes);
+    char* base = nullptr;
+    GF2C_CUDA(cudaMalloc((void**)&base, total));
+    b->allocs.push_back(base);
+    for (const Part& p : parts) {
+      GF2C_CUDA(cudaMemcpy(base, p.src, p.bytes, cudaMemcpyHostToDevice));
+      *p.out = base;
+      base += padded(p.bytes);
+    }
+    return GF2C_OK;
+  }
+};
 
 template <int T>
 size_t enc_smem() { return syn_smem_bytes<T>() + kBchWarps * 8 * 4 + kBchWarps * 16 * 2; }
@@ -862,15 +880,18 @@ int bch_upload(gf2c_bch* b) {
   GF2C_CUDA(cudaGetDevice(&dev));
   if (b->dev == dev) return GF2C_OK;
   if (b->dev >= 0) return set_error(GF2C_ERR_UNSUPPORTED, "BCH code already bound to another device");
-  int rc;
-  const uint64_t* quad = nullptr;
-  if ((rc = dev_upload(b, b->h_exp, &b->d.exp)) || (rc = dev_upload(b, b->h_log, &b->d.log)) ||
-      (rc = dev_upload(b, b->h_half, &b->d.half)) || (rc = dev_upload(b, b->h_lane_mul, &b->d.lane_mul)) ||
-      (rc = dev_upload(b, b->h_lane_out, &b->d.lane_out)) ||
-      (rc = dev_upload(b, b->h_quad, &quad)) || (rc = dev_upload(b, b->h_mul, &b->d.mul)) ||
-      (rc = dev_upload(b, b->h_lf, &b->d.lf)) || (rc = dev_upload(b, b->h_acol, &b->d.acol)))
-    return rc;
-  b->d.quad = (const uint2*)quad;
+  BchUpload up;
+  up.add(b->h_exp, &b->d.exp);
+  up.add(b->h_log, &b->d.log);
+  up.add(b->h_half, &b->d.half);
+  up.add(b->h_lane_mul, &b->d.lane_mul);
+  up.add(b->h_lane_out, &b->d.lane_out);
+  up.add(b->h_quad, &b->d.quad);
+  up.add(b->h_mul, &b->d.mul);
+  up.add(b->h_lf, &b->d.lf);
+  up.add(b->h_acol, &b->d.acol);
+  int rc = up.run(b);
+  if (rc) return rc;
   GF2C_CUDA(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
   if ((rc = b->d.t == 12 ? set_kernel_attrs<12>(b) : set_kernel_attrs<10>(b))) return rc;
   if (b->sliced) {
@@ -1059,12 +1080,15 @@ int gf2c_bch_create_dvbt2(int32_t frame_size, int32_t rate, gf2c_bch** out) {
     };
     const uint32_t back = apow(-j), fin = apow(j * (d.n - 1 - 32ll * (slice_steps(d.n) - 1)));
     for (int half = 0; half < 2; half++)
-      for (int v = 0; v < 256; v++) {
-        uint32_t x = 0;
-        for (int e = 0; e < 8 && 8 * half + e < d.m; e++)
-          if (v >> e & 1) x ^= apow(32 * j * (8 * half + e));
-        b->h_lane_mul[(size_t)s * 512 + 256 * half + v] = (uint16_t)vec_of(mul(x, back));
-        b->h_lane_out[(size_t)s * 512 + 256 * half + v] = (uint16_t)mul(x, fin);
+      for (int e = 0; e < 8 && 8 * half + e < d.m; e++) {  // linear: powers of two, then sums
+        const uint32_t x = apow(32 * j * (8 * half + e));
+        uint16_t* lm = &b->h_lane_mul[(size_t)s * 512 + 256 * half];
+        uint16_t* lo = &b->h_lane_out[(size_t)s * 512 + 256 * half];
+        const uint16_t xm = (uint16_t)vec_of(mul(x, back)), xo = (uint16_t)mul(x, fin);
+        for (int v = 0; v < 1 << e; v++) {
+          lm[(1 << e) + v] = lm[v] ^ xm;
+          lo[(1 << e) + v] = lo[v] ^ xo;
+        }
       }
   }
   // parity from odd syndromes: P[b][q] = bit (b % m) of S_(2(b/m)+1) of parity bit q

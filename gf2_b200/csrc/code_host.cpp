@@ -616,19 +616,36 @@ int prepare_encoder(HostCode& c) {
   return GF2C_OK;
 }
 
-template <class T>
-static int dev_copy(HostCode& c, const std::vector<T>& v, const T** out) {
-  if (v.empty()) {
-    *out = nullptr;
+// Tables of one upload, in one device allocation with 256-byte aligned parts (an
+// allocation per table, two dozen of them, made most of a code's first call).
+struct TableUpload {
+  struct Part {
+    const void* src;
+    size_t bytes;
+    const void** out;
+  };
+  std::vector<Part> parts;
+  template <class T>
+  void add(const std::vector<T>& v, const T** out) {
+    parts.push_back(Part{v.data(), sizeof(T) * v.size(), (const void**)out});
+  }
+  int run(HostCode& c) {
+    auto padded = [](size_t x) { return (x + 255) / 256 * 256; };
+    size_t total = 0;
+    for (const Part& p : parts) total += padded(p.bytes);
+    char* base = nullptr;
+    if (total) {
+      GF2C_CUDA(cudaMalloc((void**)&base, total));
+      c.dev_allocs.push_back(base);
+    }
+    for (const Part& p : parts) {
+      if (p.bytes) GF2C_CUDA(cudaMemcpy(base, p.src, p.bytes, cudaMemcpyHostToDevice));
+      *p.out = p.bytes ? base : nullptr;
+      base += padded(p.bytes);
+    }
     return GF2C_OK;
   }
-  void* p = nullptr;
-  GF2C_CUDA(cudaMalloc(&p, sizeof(T) * v.size()));
-  c.dev_allocs.push_back(p);
-  GF2C_CUDA(cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
-  *out = (const T*)p;
-  return GF2C_OK;
-}
+};
 
 int upload_code(HostCode& c) {
   std::lock_guard<std::mutex> lock(c.dev_mu);
@@ -656,53 +673,56 @@ int upload_code(HostCode& c) {
     d.max_nchk = c.max_nchk;
     d.lay_dvb = layered_dvb_bucket(c);
     for (uint32_t x : c.cg_sync) d.lay_runs = std::max(d.lay_runs, __builtin_popcount(x | x << 1));
-    int rc;
-    if ((rc = dev_copy(c, c.cg, &d.cg))) return rc;
-    if ((rc = dev_copy(c, c.cg_sync, &d.cg_sync))) return rc;
-    if ((rc = dev_copy(c, c.slot_var, &d.slot_var))) return rc;
-    if ((rc = dev_copy(c, c.chk_cg, &d.chk_cg))) return rc;
-    if ((rc = dev_copy(c, c.vg, &d.vg))) return rc;
-    if ((rc = dev_copy(c, c.vg_slot, &d.vg_slot))) return rc;
-    if ((rc = dev_copy(c, c.vg_chk, &d.vg_chk))) return rc;
-    if ((rc = dev_copy(c, c.vg_ci, &d.vg_ci))) return rc;
-    if ((rc = dev_copy(c, c.slot_desc, &d.slot_desc))) return rc;
-    if ((rc = dev_copy(c, c.slot_desc.empty() ? std::vector<int>() : c.cg_ninfo, &d.cg_ninfo))) return rc;
+    TableUpload up;
+    up.add(c.cg, &d.cg);
+    up.add(c.cg_sync, &d.cg_sync);
+    up.add(c.slot_var, &d.slot_var);
+    up.add(c.chk_cg, &d.chk_cg);
+    up.add(c.vg, &d.vg);
+    up.add(c.vg_slot, &d.vg_slot);
+    up.add(c.vg_chk, &d.vg_chk);
+    up.add(c.vg_ci, &d.vg_ci);
+    up.add(c.slot_desc, &d.slot_desc);
+    if (!c.slot_desc.empty()) up.add(c.cg_ninfo, &d.cg_ninfo);
     d.z = c.slot_desc.empty() ? 0 : c.z;
-    if ((rc = dev_copy(c, c.sp_cg, &d.sp_cg))) return rc;
-    if ((rc = dev_copy(c, c.sp_desc, &d.sp_desc))) return rc;
-    if ((rc = dev_copy(c, c.sp_absent, &d.sp_absent))) return rc;
-    if ((rc = dev_copy(c, c.sp_cchunk, &d.sp_cchunk))) return rc;
-    if ((rc = dev_copy(c, c.sp_vg, &d.sp_vg))) return rc;
-    if ((rc = dev_copy(c, c.sp_ci, &d.sp_ci))) return rc;
-    if ((rc = dev_copy(c, c.sp_vchunk, &d.sp_vchunk))) return rc;
-    if ((rc = dev_copy(c, c.sp_u2v, &d.sp_u2v))) return rc;
+    up.add(c.sp_cg, &d.sp_cg);
+    up.add(c.sp_desc, &d.sp_desc);
+    up.add(c.sp_absent, &d.sp_absent);
+    up.add(c.sp_cchunk, &d.sp_cchunk);
+    up.add(c.sp_vg, &d.sp_vg);
+    up.add(c.sp_ci, &d.sp_ci);
+    up.add(c.sp_vchunk, &d.sp_vchunk);
+    up.add(c.sp_u2v, &d.sp_u2v);
     d.sp_ncchunk = (int)c.sp_cchunk.size();
     d.sp_nvchunk = (int)c.sp_vchunk.size();
     d.sp_mode = c.sp_mode;
     d.sp_nvd = (int)c.sp_vd.size();
     d.sp_ndesc = (int)c.sp_desc.size();
-    if ((rc = dev_copy(c, c.sp_vh, &d.sp_vh))) return rc;
-    if ((rc = dev_copy(c, c.sp_vd, &d.sp_vd))) return rc;
-    if ((rc = dev_copy(c, c.sp_rot, &d.sp_rot))) return rc;
-    if ((rc = dev_copy(c, c.sp_ve, &d.sp_ve))) return rc;
+    up.add(c.sp_vh, &d.sp_vh);
+    up.add(c.sp_vd, &d.sp_vd);
+    up.add(c.sp_rot, &d.sp_rot);
+    up.add(c.sp_ve, &d.sp_ve);
     std::vector<int> rp(c.row_ptr.begin(), c.row_ptr.end()), ri(c.row_idx.begin(), c.row_idx.end());
-    if ((rc = dev_copy(c, rp, &d.csr_ptr))) return rc;
-    if ((rc = dev_copy(c, ri, &d.csr_idx))) return rc;
+    up.add(rp, &d.csr_ptr);
+    up.add(ri, &d.csr_idx);
     d.enc_kind = c.kind == 2 ? 0 : 1;
     if (c.kind == 2) {
       d.enc_q = c.q;
       d.enc_rg_total = (int)c.enc_rg_ent.size();
-      if ((rc = dev_copy(c, c.enc_rg_ptr, &d.enc_rg_ptr))) return rc;
-      if ((rc = dev_copy(c, c.enc_rg_ent, &d.enc_rg_ent))) return rc;
+      up.add(c.enc_rg_ptr, &d.enc_rg_ptr);
+      up.add(c.enc_rg_ent, &d.enc_rg_ent);
     }
+    int rc = up.run(c);
+    if (rc) return rc;
     c.dev = d;
     c.dev_id = dev;
   }
   if (need_enc) {
-    int rc;
-    if ((rc = dev_copy(c, c.enc_p, &c.dev.enc_p))) return rc;
-    if ((rc = dev_copy(c, c.enc_msg_cols, &c.dev.enc_msg_cols))) return rc;
-    if ((rc = dev_copy(c, c.enc_par_cols, &c.dev.enc_par_cols))) return rc;
+    TableUpload up;
+    up.add(c.enc_p, &c.dev.enc_p);
+    up.add(c.enc_msg_cols, &c.dev.enc_msg_cols);
+    up.add(c.enc_par_cols, &c.dev.enc_par_cols);
+    if (int rc = up.run(c)) return rc;
   }
   return GF2C_OK;
 }
