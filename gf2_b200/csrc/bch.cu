@@ -859,9 +859,8 @@ size_t syn_smem() { return syn_smem_bytes<T>() + kBchWarps * 32 * 2; }
 
 template <int T>
 int set_kernel_attrs(gf2c_bch* b) {
-  GF2C_CUDA(cudaFuncSetAttribute(bch_encode_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)enc_smem<T>()));
-  GF2C_CUDA(cudaFuncSetAttribute(bch_syndrome_bm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)syn_smem<T>()));
+  GF2C_CUDA(allow_smem((const void*)bch_encode_kernel<T>, enc_smem<T>()));
+  GF2C_CUDA(allow_smem((const void*)bch_syndrome_bm_kernel<T>, syn_smem<T>()));
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ_enc, bch_encode_kernel<T>, kBchWarps * 32,
                                                           enc_smem<T>()));
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ_syn, bch_syndrome_bm_kernel<T>, kBchWarps * 32,
@@ -898,7 +897,7 @@ int bch_upload(gf2c_bch* b) {
     const void* k = slice_kernel(b->d.t, b->d.m);
     const int sm = (int)(b->d.t == 12 ? slice_smem_bytes<12>() : slice_smem_bytes<10>());
     if (k) {
-      GF2C_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+      GF2C_CUDA(allow_smem(k, sm));
       GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ_slice, k, kSliceThreads, sm));
       GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &b->occ_loc, b->d.t == 12 ? (const void*)bch_locator_kernel<12> : (const void*)bch_locator_kernel<10>,
@@ -907,7 +906,7 @@ int bch_upload(gf2c_bch* b) {
     }
   }
   const int chien_smem = (b->d.N + kChienOff) * 2;
-  GF2C_CUDA(cudaFuncSetAttribute(bch_chien_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, chien_smem));
+  GF2C_CUDA(allow_smem((const void*)bch_chien_kernel, chien_smem));
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ_chien, bch_chien_kernel, kChienThreads, chien_smem));
   b->occ_enc = std::max(b->occ_enc, 1);
   b->occ_syn = std::max(b->occ_syn, 1);

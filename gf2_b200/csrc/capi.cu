@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <tuple>
 
 #include "internal.h"
@@ -23,6 +24,20 @@ int set_error(int code, const std::string& msg) {
 int cuda_error(cudaError_t e, const char* what) {
   g_error = std::string(what) + ": " + cudaGetErrorString(e);
   return GF2C_ERR_CUDA;
+}
+
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limits;  // per device and kernel
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& limit = limits[{dev, kernel}];
+  if (bytes <= limit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit = bytes;
+  return e;
 }
 
 // Device buffer that only grows.
@@ -568,7 +583,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     GF2C_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->dev));
     const size_t with = (size_t)d->lay_dbuf_off + (size_t)d->lay_dbuf_floats * 4;
     if (with <= (size_t)optin) {
-      GF2C_CUDA(cudaFuncSetAttribute(d->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)with));
+      GF2C_CUDA(allow_smem(d->kernel, with));
       GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ0, d->kernel, threads, d->smem));
       GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, d->kernel, threads, with));
     }
@@ -603,10 +618,10 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     const size_t off = (d->smem + 15) & ~(size_t)15, with = off + 2 * mx + 16;
     if (k && with <= (size_t)optin) {
       if (d->kernel) {
-        GF2C_CUDA(cudaFuncSetAttribute(d->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
+        GF2C_CUDA(allow_smem(d->kernel, d->smem));
         GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ0, d->kernel, threads, d->smem));
       }
-      GF2C_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)with));
+      GF2C_CUDA(allow_smem(k, with));
       GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, k, threads, with));
       if (occ1 > 0 && (occ1 >= occ0 || !d->kernel || std::getenv("GF2C_FORCE_STAGE"))) {
         d->kernel = k;
@@ -619,7 +634,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   if (!d->kernel)
     return set_error(GF2C_ERR_UNSUPPORTED, "no decode kernel for this configuration (several checks per thread "
                                           "need the staged kernel: 16-byte aligned row groups, >= 3 row groups)");
-  GF2C_CUDA(cudaFuncSetAttribute(d->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
+  GF2C_CUDA(allow_smem(d->kernel, d->smem));
   int occ = 0;
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, d->kernel, threads, d->smem));
   if (occ <= 0) return set_error(GF2C_ERR_UNSUPPORTED, "decode kernel does not fit on an SM with this shape");
@@ -639,7 +654,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   d->lay_few_grid = d->grid;
   if (d->lay_many_kernel) {
     int b = 0;
-    GF2C_CUDA(cudaFuncSetAttribute(d->lay_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
+    GF2C_CUDA(allow_smem(d->lay_many_kernel, d->smem));
     GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, d->lay_many_kernel, d->lay_many_threads, d->smem));
     d->lay_many_grid = sms * b;
     d->grid = std::max(d->grid, d->lay_many_grid);
@@ -659,7 +674,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
       d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, false);
       d->team_threads = state_flood_threads();
     }
-    GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->sf_team.smem));
+    GF2C_CUDA(allow_smem(d->sf_team_kernel, d->sf_team.smem));
     GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     for (int lg = 1; lg <= 4; lg++) {
       cudaLaunchAttribute at;

@@ -581,7 +581,7 @@ static int launch_encode_dvb(const DevCode* dcode, const DevCode& h, const uint6
   const size_t smem =
       (size_t)(((2 * h.words_k * G + 3) & ~3) + dvbt2_scratch_words(h.k / 360, h.enc_q, h.m, h.enc_rg_total, G)) * 4;
   int per_sm = 1;
-  GF2C_CUDA(cudaFuncSetAttribute(encode_dvb_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)encode_dvb_kernel<G>, smem));
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_dvb_kernel<G>, kEncodeThreads, smem));
   const long long grid = std::min<long long>((frames + G - 1) / G, (long long)sms * std::max(per_sm, 1));
   encode_dvb_kernel<G><<<(int)grid, kEncodeThreads, smem, st>>>(dcode, msg, frames, cw);
@@ -608,7 +608,7 @@ int launch_encode(const DevCode* dcode, const DevCode& h, const uint64_t* msg, l
     return frames >= 8ll * sms ? launch_encode_dvb<4>(dcode, h, msg, frames, cw, sms, st)
                                : launch_encode_dvb<1>(dcode, h, msg, frames, cw, sms, st);
   size_t smem = encode_smem(h);
-  GF2C_CUDA(cudaFuncSetAttribute(encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)encode_kernel, smem));
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_kernel, 256, smem));
   const long long grid = std::max<long long>(1, std::min<long long>(frames, (long long)sms * std::max(per_sm, 1)));
   encode_kernel<<<(int)grid, 256, smem, st>>>(dcode, msg, frames, cw);
@@ -621,7 +621,7 @@ int launch_syndrome(const DevCode* dcode, const DevCode& h, const uint64_t* cw, 
   if (frames <= 0) return GF2C_OK;
   size_t smem = (size_t)((h.n + 31) / 32) * 4;
   if (h.enc_kind == 0) smem += (size_t)dvbt2_scratch_words(h.k / 360, h.enc_q, h.m, h.enc_rg_total, 1) * 4;
-  GF2C_CUDA(cudaFuncSetAttribute(syndrome_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)syndrome_kernel, smem));
   syndrome_kernel<<<grid_for(frames), 256, smem, st>>>(dcode, cw, frames, synd, weight);
   GF2C_CUDA(cudaGetLastError());
   return GF2C_OK;
@@ -632,7 +632,7 @@ int launch_channel(const DevCode* dcode, const DevCode& h, uint64_t seed, uint64
                    cudaStream_t st) {
   if (frames <= 0) return GF2C_OK;
   size_t smem = encode_smem(h);
-  GF2C_CUDA(cudaFuncSetAttribute(channel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)channel_kernel, smem));
   uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   channel_kernel<<<grid_for(frames), kEncThreads, smem, st>>>(dcode, key, frame0, frames, sigma2, info, cw, llr);
   GF2C_CUDA(cudaGetLastError());

@@ -177,6 +177,13 @@ int cuda_error(cudaError_t e, const char* what);
     if (_e != cudaSuccess) return ::gf2c::cuda_error(_e, #call); \
   } while (0)
 
+// Lets launches of `kernel` on the current device take `bytes` of dynamic shared
+// memory.  The limit is the kernel's, shared by every decoder, code and thread
+// that launches it, so it is only ever raised: a smaller code's setup must not
+// take it away from a larger one's launches.  For shared memory whose size
+// depends on the code, this stands in place of cudaFuncSetAttribute.
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+
 // host code construction (code_host.cpp)
 int build_dvbt2(int frame, int rate, HostCode& c);
 int build_qc(const int32_t* base, int mb, int nb, int z, HostCode& c);

@@ -383,8 +383,8 @@ static int launch_dvb(const DevCode* dcode, const DevCode& h, int T, int L, cons
                       long long frames, const float* alpha, const float* beta, float* X, float* B, char* work,
                       long long work_stride, int grid, float* pf, cudaStream_t st) {
   const size_t smem = train_smem(h);
-  GF2C_CUDA(cudaFuncSetAttribute(nms_dvb_forward_kernel<D, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GF2C_CUDA(cudaFuncSetAttribute(nms_dvb_backward_kernel<D, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)nms_dvb_forward_kernel<D, PART>, smem));
+  GF2C_CUDA(allow_smem((const void*)nms_dvb_backward_kernel<D, PART>, smem));
   nms_dvb_forward_kernel<D, PART><<<grid, kTrainThreads, smem, st>>>(dcode, T, L, llr, cw, frames, alpha, beta, (uint4*)X,
                                                                      B, work, work_stride, pf);
   GF2C_CUDA(cudaGetLastError());

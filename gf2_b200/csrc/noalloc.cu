@@ -204,7 +204,7 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
   // launch attributes and occupancy, set up again only when the kernel or its
   // shared memory changes (the first call on a device does it)
   if (S.kern != kern || S.kern_smem != smem) {
-    GF2C_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GF2C_CUDA(allow_smem(kern, smem));
     int occ = 0;
     GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
     if (occ <= 0) return set_error(GF2C_ERR_UNSUPPORTED, "decode kernel does not fit on an SM");

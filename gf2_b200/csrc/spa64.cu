@@ -286,7 +286,7 @@ extern "C" int gf2c_judge_spa64(const gf2c_code* code, int32_t schedule, const f
   a.app_off = msg_bytes;
   const int threads = std::max(32, (h.max_nchk + 31) / 32 * 32);
   const size_t smem = (size_t)((h.n + 31) / 32) * 4;
-  GF2C_CUDA(cudaFuncSetAttribute(spa64_judge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF2C_CUDA(allow_smem((const void*)spa64_judge_kernel, smem));
   spa64_judge_kernel<<<grid, threads, smem, st>>>(a);
   GF2C_CUDA(cudaGetLastError());
   return GF2C_OK;
