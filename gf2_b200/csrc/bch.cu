@@ -476,8 +476,16 @@ __device__ __forceinline__ uint32_t word_mask(int bits, int w) {
   return left >= 32 ? ~0u : left > 0 ? (1u << left) - 1u : 0u;
 }
 
+// Barrier of a sliced CTA's warps.  They meet from different instances of
+// sliced_pass, where __syncthreads() may not stand: it asks every thread of the
+// CTA to reach the same barrier of the source.  A PTX barrier counts the threads
+// that arrive at its number, wherever they arrive from.
+__device__ __forceinline__ void slice_sync() {
+  asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(kSliceThreads) : "memory");
+}
+
 // One warp's factors over the whole frames; every warp of the CTA takes the same
-// barriers.
+// number of barriers.
 template <int M, int FIRST, int COUNT>
 __device__ __forceinline__ void sliced_pass(const BchDev& B, const uint64_t* __restrict__ cw,
                                             uint64_t* __restrict__ msg, long long f0, int nf, uint32_t* planes,
@@ -505,10 +513,10 @@ __device__ __forceinline__ void sliced_pass(const BchDev& B, const uint64_t* __r
       if (i < rows && w < wout) out[(long long)i * wout + 32 * blk] = x[i] & mk;
     }
     if (blk + 1 < blocks) fetch(blk + 1);
-    __syncthreads();  // tile written; the last block's planes read
+    slice_sync();  // tile written; the last block's planes read
 #pragma unroll
     for (int i = 0; i < 8; i++) planes[(8 * warp + i) * 32 + lane] = tr(tile[lane * kTilePitch + 8 * warp + i]);
-    __syncthreads();  // planes written, tile read
+    slice_sync();  // planes written, tile read
 #pragma unroll 1
     for (int w0 = 0; w0 < 32; w0 += 8) {
       uint32_t b[8];
