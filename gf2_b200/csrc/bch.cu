@@ -596,23 +596,27 @@ __device__ __forceinline__ uint32_t mod_n(const BchDev& B, uint32_t x) {
   return x >= N ? x - N : x;
 }
 
-// Scans position steps from s on for roots of a locator of degree D whose
-// coefficients (logarithms, lane j holds coefficient j) are all nonzero, up to
-// the first segment of kChienSeg steps that holds one or the end.  Returns this
-// lane's root steps in that segment (s then is the step behind it).  sexp[x] =
+// Scans position steps from s on for roots of a locator of degree D (logarithms
+// of its coefficients, lane j holds coefficient j; with ZEROS some may be zero),
+// up to the first segment of kChienSeg steps that holds one or the end.  Returns
+// this lane's root steps in that segment (s then is the step behind it).  sexp[x] =
 // alpha^(x - kChienOff); term j keeps Ep = (its exponent mod N) + kChienOff,
 // which stays in [0, N + kChienOff) over a segment of steps of -32 j each, so
 // the steps inside a segment are constant offsets of the load and the
 // reduction mod N happens once per segment.
-template <int D>
+template <int D, bool ZEROS>
 __device__ __forceinline__ uint32_t chien_scan(const BchDev& B, const uint16_t* __restrict__ sexp, uint32_t myL,
                                                int lane, int& s) {
   const uint32_t N = (uint32_t)B.N;
   const int steps = (B.n + 31) >> 5;
-  uint32_t Ep[D];
+  uint32_t Ep[D], keep[ZEROS ? D : 1];  // keep: which terms are there
 #pragma unroll
   for (int j = 1; j <= D; j++) {
-    const uint32_t Lj = __shfl_sync(0xffffffffu, myL, j);
+    uint32_t Lj = __shfl_sync(0xffffffffu, myL, j);
+    if (ZEROS) {
+      keep[ZEROS ? j - 1 : 0] = Lj == kLogZero ? 0u : 0xffffu;
+      Lj = Lj == kLogZero ? 0u : Lj;
+    }
     const uint32_t back = mod_n(B, (uint32_t)j * (uint32_t)(32 * s + lane));
     Ep[j - 1] = (Lj >= back ? Lj - back : Lj + N - back) + kChienOff;
   }
@@ -624,7 +628,10 @@ __device__ __forceinline__ uint32_t chien_scan(const BchDev& B, const uint16_t* 
       for (int g = 0; g < kChienUnroll; g++) {
         uint32_t acc = 0;
 #pragma unroll
-        for (int j = 1; j <= D; j++) acc ^= sexp[Ep[j - 1] - 32u * j * g];
+        for (int j = 1; j <= D; j++) {
+          const uint32_t v = sexp[Ep[j - 1] - 32u * j * g];
+          acc ^= ZEROS ? v & keep[ZEROS ? j - 1 : 0] : v;
+        }
         const int i = 32 * (s + g0 + g) + lane;
         hit |= (uint32_t)(acc == 1u && i < B.n) << (g0 + g);
       }
@@ -753,13 +760,18 @@ __global__ void __launch_bounds__(kChienThreads, 1) bch_chien_kernel(const BchDe
     uint64_t* mo = msg + f * B.words_k;
     int roots = 0, st = 0, deg = bk == 0 ? degs[f] : bk;
     uint32_t L = lane <= deg ? myL : (uint32_t)kLogZero;
-    bool plain = bk != 0;  // every coefficient nonzero, at most kChienFastMax of them
     const int steps = (B.n + 31) >> 5;
-    while (plain && deg > 2 && st < steps) {
+    while (bk != 0 && deg > 2 && st < steps) {
+      // A locator whose root is divided out may get a zero coefficient (about one
+      // frame in 1000).  It is scanned with its terms masked; the general evaluator
+      // takes several times as long, and a batch of one wave waits for such a frame
+      // (4700 normal 1/2 frames of 15 errors: 688 us with it, 537 us).
+      const bool zeros = __any_sync(0xffffffffu, lane >= 1 && lane <= deg && L == kLogZero);
       uint32_t hit = 0;
-      switch (deg) {
-#define GF2C_SCAN(D) \
-  case D: hit = chien_scan<D>(B, sexp, L, lane, st); break
+      switch (deg + (zeros ? 16 : 0)) {
+#define GF2C_SCAN(D)                                                    \
+  case D: hit = chien_scan<D, false>(B, sexp, L, lane, st); break;      \
+  case D + 16: hit = chien_scan<D, true>(B, sexp, L, lane, st); break
         GF2C_SCAN(3);
         GF2C_SCAN(4);
         GF2C_SCAN(5);
@@ -769,8 +781,8 @@ __global__ void __launch_bounds__(kChienThreads, 1) bch_chien_kernel(const BchDe
         GF2C_SCAN(9);
         GF2C_SCAN(10);
         GF2C_SCAN(11);
-        GF2C_SCAN(12);
 #undef GF2C_SCAN
+        case 12: hit = chien_scan<12, false>(B, sexp, L, lane, st); break;
       }
       // divide the roots of this segment out
       for (uint32_t who = __ballot_sync(0xffffffffu, hit != 0u); who; who &= who - 1) {
@@ -783,10 +795,9 @@ __global__ void __launch_bounds__(kChienThreads, 1) bch_chien_kernel(const BchDe
           deg--;
         }
       }
-      plain = !__any_sync(0xffffffffu, lane >= 1 && lane <= deg && L == kLogZero);
     }
     if (deg >= 1 && st < steps) {
-      if (deg <= 2 && bk != 0)
+      if (bk != 0)
         roots += chien_close(B, sexp, deg, __shfl_sync(0xffffffffu, L, 1), __shfl_sync(0xffffffffu, L, 2), 32 * st, lane,
                              mo);
       else
