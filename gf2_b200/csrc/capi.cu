@@ -90,6 +90,12 @@ struct gf2c_decoder {
   // more registers, and short frames lose: 2048 normal 3/5 frames 59 -> 72 ms).
   const void* lay_many_kernel = nullptr;
   int lay_many_threads = 0, lay_many_grid = 0, lay_few_grid = 0;
+  // Frames in flight of the plain launch shape: what a chunk of the host-memory
+  // pipelines holds at least.  The larger grids of the shapes above and below
+  // would make the chunks too few to overlap copies and decoding (learned decoder
+  // with fallback, 1500 normal 2/3 frames from pinned memory: 10.3 ms in chunks of
+  // 296 frames and more, 15.3 ms in chunks of 592).
+  int wave = 0;
   bool state_flood = false;  // check-state flooding min-sum kernel (state_flood.cu)
   int sf_app_soff = 0, sf_tab_off = -1;
   // check-state kernel, frame state on chip: CTAs of 1024, 512 and 256 threads
@@ -639,7 +645,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, d->kernel, threads, d->smem));
   if (occ <= 0) return set_error(GF2C_ERR_UNSUPPORTED, "decode kernel does not fit on an SM with this shape");
   int bps = o.blocks_per_sm ? std::min(o.blocks_per_sm, occ) : occ;
-  d->grid = sms * bps;
+  d->grid = d->wave = sms * bps;
   if (d->state_flood && d->sf_tab_off >= 0 && d->sf_st_off == d->sf_app_off && o.threads_per_block == 0 &&
       o.blocks_per_sm == 0) {
     // Small codes leave most of a 1024-thread CTA's warps waiting at the two
@@ -982,15 +988,15 @@ int gf2c_decode_batch(gf2c_decoder* dec, const float* llr, int64_t frames, int32
   // frame queue).  Only the last chunk is decoded hardest frames first: the
   // ordering kernels of the others would wait for those SMs, which the next
   // chunk's decode fills anyway.
-  const int64_t chunk = std::max<int64_t>(dec->grid, (frames + 7) / 8);
+  const int64_t chunk = std::max<int64_t>(dec->wave, (frames + 7) / 8);
   if (frames >= 2 * chunk && bl >= ((size_t)64 << 20) && pipeline_ready(dec)) {
     GF2C_CUDA(cudaEventRecord(dec->pev_fork, st));
     GF2C_CUDA(cudaStreamWaitEvent(dec->pstream, dec->pev_fork, 0));
     GF2C_CUDA(cudaStreamWaitEvent(dec->cstream, dec->pev_fork, 0));
     int chunks = 0, launches = 0;
-    const int64_t csz = even_chunk(frames, dec->grid);
+    const int64_t csz = even_chunk(frames, dec->wave);
     for (int64_t f0 = 0, nf = 0; f0 < frames; f0 += nf, chunks++) {
-      nf = chunk_frames(csz, frames - f0, dec->grid);
+      nf = chunk_frames(csz, frames - f0, dec->wave);
       const int slot = chunks & 1;
       cudaStream_t s = slot ? dec->pstream : st;
       const size_t ln = (size_t)nf * h.n * 4, lo = (size_t)f0 * h.n * 4;
@@ -1170,7 +1176,7 @@ int gf2c_decode_batch_fallback(gf2c_decoder* primary, gf2c_decoder* fallback, co
       (rc = primary->s_so.ensure((size_t)frames)) || (rc = primary->fb_list.ensure((size_t)frames * 8)) ||
       (rc = primary->fb_count.ensure(64 * 8)))
     return rc;
-  const int64_t wave = std::max(primary->grid, fallback->grid);
+  const int64_t wave = std::max(primary->wave, fallback->wave);
   const bool pipe = frames >= 3 * wave && bl >= ((size_t)64 << 20) && pipeline_ready(primary) &&
                     (fallback == primary || fallback_stream_ready(primary));
   const bool fsplit = pipe && fallback != primary;
@@ -1354,7 +1360,7 @@ int gf2c_decode_mixed(gf2c_decoder* dec, const float* llr, const int64_t* llr_of
   // gf2c_decode_batch).  The frame order of a chunk (code by code, longest
   // codes first, then by frame index, the ordering kernel's rule) is made on
   // the host; the persistent kernel takes the chunk's frames from it.
-  const int64_t wave = dec->grid;
+  const int64_t wave = dec->wave;
   if (ordered && frames >= 3 * wave && (size_t)llr_total * 4 >= ((size_t)64 << 20) && pipeline_ready(dec) &&
       dec->s_cnt.ensure(64 * 8) == GF2C_OK) {
     std::vector<int64_t> mem((size_t)frames), ord((size_t)frames);

@@ -101,3 +101,15 @@ def test_fallback_same_decoder_host_pipeline(gpu):
     assert h["fallback_count"] == int(d["fallback_count"][0])
     for k in ("msg", "iters", "conv", "synd_ok"):
         assert torch.equal(h[k], d[k].cpu()), k
+
+
+def test_fallback_host_batch_of_a_few_waves_is_pipelined(gpu):
+    """1000 normal frames from host memory go in three chunks (296 frames fill the
+    GPU), each with its primary and its fallback pass, not in one piece."""
+    code = g.LdpcCode.dvb_t2_normal(g.CodeRate.Rate2_3)
+    L, T = code.layers(), 2
+    prim = g.LdpcDecoder(code, algorithm=g.ALGO_NMS, schedule=g.SCHED_LAYERED, msg_dtype=g.MSG_F16,
+                         nms_alpha=np.full((T, L), 0.8, np.float32), nms_beta=np.zeros((T, L), np.float32))
+    fb = g.LdpcDecoder(code, algorithm=g.ALGO_SPA_FAST, schedule=g.SCHED_LAYERED, msg_dtype=g.MSG_F16)
+    prim.decode_with_fallback(fb, torch.full((1000, code.n()), 4.0).numpy(), T, 2)
+    assert prim.last_launches() >= 3 * 3  # a decode, a list and a fallback decode per chunk
