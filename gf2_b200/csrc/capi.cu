@@ -500,7 +500,22 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   d->work_stride = c2v_bytes + (need_gapp ? ((long long)d->max_n * 4 + 255) / 256 * 256 : 0);
   d->kernel = layered ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads)
                       : flood_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads);
-  if (multi_mixed && d->dcmax <= 22) d->kernel = layered_kernel_ptr(o.algorithm, o.msg_dtype, 0, threads);
+  // A mixed batch of codes of different slot counts: the kernel that runs each
+  // frame with its own code's count, where there is one (SFU sum-product, up to
+  // 22 slots); in the kernel of the largest count every check of a smaller code
+  // computes the slots beyond its own (short 1/2 with a 13-slot QC code, 4096
+  // frames: 5.9 against 7.4 ms; at 192 threads 7.6 against 24 ms).
+  if (layered && threads <= 384) {
+    bool differ = false, dispatchable = true;
+    for (auto* c : d->codes) {
+      const int b = layered_dcmax_bucket(c->h->max_dc);
+      differ = differ || b != d->dcmax;
+      dispatchable = dispatchable && b > 0 && b <= 22;
+    }
+    const void* k = ((differ || multi_mixed) && dispatchable) ? layered_kernel_ptr(o.algorithm, o.msg_dtype, 0, threads)
+                                                               : nullptr;
+    if (k) d->kernel = k;
+  }
   // DVB-T2 codes with a fused-row algorithm: their own kernels, one code or a
   // mixed batch.  Shared memory: bitmap, posteriors (short frames), the deltas
   // of the slots inside runs of one block, the tables.

@@ -632,9 +632,10 @@ static const void* dvb_exact(int D, bool shared_app) {
 template <int ALGO, int MSG16>
 static const void* dvb_t(int D, bool shared_app, int threads) {
   if (D == 0) {
-    if constexpr (ALGO == L_SPA_FAST && MSG16) {
+    if constexpr (ALGO == L_SPA_FAST) {
       if (threads == 384) return (const void*)bp_layered_dvb_kernel<ALGO, MSG16, 0, 384, 2, PL_SHARED, false>;
-      if (threads == 192) return (const void*)bp_layered_dvb_kernel<ALGO, MSG16, 0, 192, 4, PL_GLOBAL, false>;
+      if constexpr (MSG16)
+        if (threads == 192) return (const void*)bp_layered_dvb_kernel<ALGO, MSG16, 0, 192, 4, PL_GLOBAL, false>;
     }
     return nullptr;
   }

@@ -985,7 +985,25 @@ __global__ void __launch_bounds__(MAXT, MINB) bp_layered_kernel(const DecodeArgs
     }
     __syncthreads();
     int it = 0, converged = 0;
-    layered_iterations<ALGO, MSG16, DCMAX, STG, (MAXT < 384)>(a, C, app, c2v, S, maxit, it, converged, stg, &s_abort);
+    if constexpr (DCMAX > 0) {
+      layered_iterations<ALGO, MSG16, DCMAX, STG, (MAXT < 384)>(a, C, app, c2v, S, maxit, it, converged, stg,
+                                                               &s_abort);
+    } else {  // mixed batch: the exact slot count of this frame's code
+#define GF2C_LAY_CASE(D) \
+  layered_iterations<ALGO, MSG16, D, STG, (MAXT < 384)>(a, C, app, c2v, S, maxit, it, converged, stg, &s_abort)
+      switch (C.lay_bucket) {
+        case 7: GF2C_LAY_CASE(7); break;
+        case 9: GF2C_LAY_CASE(9); break;
+        case 10: GF2C_LAY_CASE(10); break;
+        case 11: GF2C_LAY_CASE(11); break;
+        case 13: GF2C_LAY_CASE(13); break;
+        case 14: GF2C_LAY_CASE(14); break;
+        case 18: GF2C_LAY_CASE(18); break;
+        case 19: GF2C_LAY_CASE(19); break;
+        default: GF2C_LAY_CASE(22); break;
+      }
+#undef GF2C_LAY_CASE
+    }
     if constexpr (STG) {
       // a copy issued for an iteration that did not run (early stop): let it land
       if (stg.pending) {
@@ -1041,6 +1059,9 @@ static const void* lay_exact(int dcmax) {
     case 22: return (const void*)bp_layered_kernel<ALGO, MSG16, 22, 384, MINB, STG>;
     case 26: return (const void*)bp_layered_kernel<ALGO, MSG16, 26, 384, MINB, STG>;
     case 32: return (const void*)bp_layered_kernel<ALGO, MSG16, 32, 384, MINB, STG>;
+    case 0:  // mixed batches: each frame runs the iterations of its code's exact slot count
+      if constexpr (ALGO == L_SPA_FAST && !STG) return (const void*)bp_layered_kernel<ALGO, MSG16, 0, 384, MINB, false>;
+      return nullptr;
   }
   return nullptr;
 }
@@ -1069,9 +1090,8 @@ static const void* lay_multi(int dcmax) {
 template <int ALGO, int MSG16>
 static const void* lay_t(int dcmax, int maxt, bool stage) {
   if (maxt > 384) return stage ? nullptr : lay_wide<ALGO, MSG16>(dcmax);
-  if (dcmax == 0) {  // a mixed batch with QC codes, two checks per thread, up to 22 slots
-    if constexpr (ALGO == L_SPA_FAST && MSG16)
-      if (maxt == 192 && !stage) return (const void*)bp_layered_kernel<ALGO, MSG16, 22, 192, 4, false>;
+  if (dcmax == 0 && maxt == 192 && !stage) {  // mixed batches, two checks per thread
+    if constexpr (ALGO == L_SPA_FAST && MSG16) return (const void*)bp_layered_kernel<ALGO, MSG16, 0, 192, 4, false>;
     return nullptr;
   }
   if constexpr (ALGO == L_SPA) {
