@@ -632,7 +632,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
       ok = ok && (states || (off % 16 == 0 && by % 16 == 0));
       if (!states) mx = std::max(mx, by);
     }
-    const void* k = ok ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads, true)
+    const void* k = ok ? layered_kernel_ptr(o.algorithm, o.msg_dtype, d->dcmax, threads, true, o.blocks_per_sm)
                        : nullptr;
     int optin = 0, occ0 = 0, occ1 = 0;
     GF2C_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->dev));

@@ -271,7 +271,8 @@ StateFloodLayout spa_flood_layout(const std::vector<const HostCode*>& codes, int
 const void* spa_flood_kernel_ptr(int algo, int msg16, int D);
 int decode_dcmax_bucket(int max_dc);
 int layered_dcmax_bucket(int max_dc);
-const void* layered_kernel_ptr(int algo, int msg16, int dcmax, int maxt, bool stage = false);
+// bps: requested CTAs per SM (0 = any); 192 threads with 5 or more picks the 64-register build
+const void* layered_kernel_ptr(int algo, int msg16, int dcmax, int maxt, bool stage = false, int bps = 0);
 // DVB-T2 layered kernels (layered_dvb.cuh): slot bucket of a code they decode
 // (0: none), and the kernel for bucket D (0: a mixed batch), the posteriors'
 // placement and 384, 192 or 128 threads (nullptr: none).

@@ -1045,23 +1045,28 @@ __global__ void __launch_bounds__(MAXT, MINB) bp_layered_kernel(const DecodeArgs
 // codes (an exact fit wastes no slot and keeps the all-edges fast path).
 // STG: the TMA-staged variant (not for the exact sum-product, which is
 // arithmetic-bound).
-template <int ALGO, int MSG16, int MINB, bool STG>
+template <int ALGO, int MSG16, int MINB, bool STG, int MAXT = 384>
 static const void* lay_exact(int dcmax) {
   switch (dcmax) {
-    case 7: return (const void*)bp_layered_kernel<ALGO, MSG16, 7, 384, MINB, STG>;
-    case 9: return (const void*)bp_layered_kernel<ALGO, MSG16, 9, 384, MINB, STG>;
-    case 10: return (const void*)bp_layered_kernel<ALGO, MSG16, 10, 384, MINB, STG>;
-    case 11: return (const void*)bp_layered_kernel<ALGO, MSG16, 11, 384, MINB, STG>;
-    case 13: return (const void*)bp_layered_kernel<ALGO, MSG16, 13, 384, MINB, STG>;
-    case 14: return (const void*)bp_layered_kernel<ALGO, MSG16, 14, 384, MINB, STG>;
-    case 18: return (const void*)bp_layered_kernel<ALGO, MSG16, 18, 384, MINB, STG>;
-    case 19: return (const void*)bp_layered_kernel<ALGO, MSG16, 19, 384, MINB, STG>;
-    case 22: return (const void*)bp_layered_kernel<ALGO, MSG16, 22, 384, MINB, STG>;
-    case 26: return (const void*)bp_layered_kernel<ALGO, MSG16, 26, 384, MINB, STG>;
-    case 32: return (const void*)bp_layered_kernel<ALGO, MSG16, 32, 384, MINB, STG>;
-    case 0:  // mixed batches: each frame runs the iterations of its code's exact slot count
-      if constexpr (ALGO == L_SPA_FAST && !STG) return (const void*)bp_layered_kernel<ALGO, MSG16, 0, 384, MINB, false>;
-      return nullptr;
+    case 7: return (const void*)bp_layered_kernel<ALGO, MSG16, 7, MAXT, MINB, STG>;
+    case 9: return (const void*)bp_layered_kernel<ALGO, MSG16, 9, MAXT, MINB, STG>;
+    case 10: return (const void*)bp_layered_kernel<ALGO, MSG16, 10, MAXT, MINB, STG>;
+    case 11: return (const void*)bp_layered_kernel<ALGO, MSG16, 11, MAXT, MINB, STG>;
+    case 13: return (const void*)bp_layered_kernel<ALGO, MSG16, 13, MAXT, MINB, STG>;
+    case 14: return (const void*)bp_layered_kernel<ALGO, MSG16, 14, MAXT, MINB, STG>;
+    case 18: return (const void*)bp_layered_kernel<ALGO, MSG16, 18, MAXT, MINB, STG>;
+    case 19: return (const void*)bp_layered_kernel<ALGO, MSG16, 19, MAXT, MINB, STG>;
+    case 22: return (const void*)bp_layered_kernel<ALGO, MSG16, 22, MAXT, MINB, STG>;
+  }
+  if constexpr (MAXT == 384) {
+    switch (dcmax) {
+      case 26: return (const void*)bp_layered_kernel<ALGO, MSG16, 26, 384, MINB, STG>;
+      case 32: return (const void*)bp_layered_kernel<ALGO, MSG16, 32, 384, MINB, STG>;
+      case 0:  // mixed batches: each frame runs the iterations of its code's exact slot count
+        if constexpr (ALGO == L_SPA_FAST && !STG)
+          return (const void*)bp_layered_kernel<ALGO, MSG16, 0, 384, MINB, false>;
+        return nullptr;
+    }
   }
   return nullptr;
 }
@@ -1078,17 +1083,14 @@ static const void* lay_wide(int dcmax) {
 }
 
 // Several checks per thread of a QC code (192 or 128 threads, 4 or 6 CTAs per
-// SM at the same 80 registers): staged FP16 kernels of the fused-row algorithms,
-// in three slot buckets (DVB-T2 codes have their own kernels, layered_dvb.cuh).
-template <int ALGO, int MSG16, int MINB, int MAXT>
-static const void* lay_multi(int dcmax) {
-  if (dcmax <= 10) return (const void*)bp_layered_kernel<ALGO, MSG16, 10, MAXT, MINB, true>;
-  if (dcmax <= 14) return (const void*)bp_layered_kernel<ALGO, MSG16, 14, MAXT, MINB, true>;
-  if (dcmax <= 22) return (const void*)bp_layered_kernel<ALGO, MSG16, 22, MAXT, MINB, true>;
-  return nullptr;
-}
+// SM at the same 80 registers): staged FP16 kernels of the fused-row algorithms
+// (DVB-T2 codes have their own kernels, layered_dvb.cuh).  192 threads with five
+// CTAs per SM: the same kernel compiled for 64 registers.  Slot counts stay exact
+// here too: in the next of three buckets (10, 14, 22) a 7-slot code took 2.32 ms
+// for 1.81, a 19-slot one 2.92 for 2.73 (2048 frames, ten iterations, 192
+// threads, SFU sum-product).
 template <int ALGO, int MSG16>
-static const void* lay_t(int dcmax, int maxt, bool stage) {
+static const void* lay_t(int dcmax, int maxt, bool stage, int bps) {
   if (maxt > 384) return stage ? nullptr : lay_wide<ALGO, MSG16>(dcmax);
   if (dcmax == 0 && maxt == 192 && !stage) {  // mixed batches, two checks per thread
     if constexpr (ALGO == L_SPA_FAST && MSG16) return (const void*)bp_layered_kernel<ALGO, MSG16, 0, 192, 4, false>;
@@ -1098,8 +1100,9 @@ static const void* lay_t(int dcmax, int maxt, bool stage) {
     return (stage || maxt < 384) ? nullptr : lay_exact<ALGO, MSG16, 1, false>(dcmax);
   } else {
     if constexpr (MSG16) {
-      if (maxt == 192) return stage ? lay_multi<ALGO, MSG16, 4, 192>(dcmax) : nullptr;
-      if (maxt == 128) return stage ? lay_multi<ALGO, MSG16, 6, 128>(dcmax) : nullptr;
+      if (maxt == 192 && bps >= 5) return stage ? lay_exact<ALGO, MSG16, 5, true, 192>(dcmax) : nullptr;
+      if (maxt == 192) return stage ? lay_exact<ALGO, MSG16, 4, true, 192>(dcmax) : nullptr;
+      if (maxt == 128) return stage ? lay_exact<ALGO, MSG16, 6, true, 128>(dcmax) : nullptr;
     }
     if (maxt < 384) return nullptr;
     return stage ? lay_exact<ALGO, MSG16, 2, true>(dcmax) : lay_exact<ALGO, MSG16, 2, false>(dcmax);

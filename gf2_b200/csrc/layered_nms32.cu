@@ -3,6 +3,6 @@
 
 namespace gf2c {
 
-const void* layered_nms32_kernel(int dcmax, int maxt, bool stage) { return lay_t<L_NMS, 0>(dcmax, maxt, stage); }
+const void* layered_nms32_kernel(int dcmax, int maxt, bool stage, int bps) { return lay_t<L_NMS, 0>(dcmax, maxt, stage, bps); }
 
 }  // namespace gf2c
