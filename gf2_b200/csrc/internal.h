@@ -35,8 +35,6 @@ struct DevCode {
   int layered_ok;                  // CGs are layers usable by the layered schedule
   int lay_bucket;                  // slot count of the layered kernel that fits this code exactly
   int max_nchk;                    // largest CG
-  int lay_dvb;                     // DVB-T2 layered kernels: slot bucket (0: not one of their codes)
-  int lay_runs;                    // most slots inside runs of one block in a row group
   const int4* cg;                  // {chk_begin, nchk, dc, edge0}
   const uint32_t* cg_sync;         // layered: bit i = barrier after slot i (dup variables)
   const int* slot_var;             // [e_slots]
@@ -70,6 +68,19 @@ struct DevCode {
   const int2* sp_vchunk;           // var chunks {var group, first j}: 32 variables of one group
   int sp_nvchunk;
   const int* sp_u2v;               // natural index of u-order variable u (nullptr: identity)
+  const int* csr_ptr;              // natural order H (m + 1)
+  const int* csr_idx;              // (nnz)
+  // encoder
+  int enc_kind;                    // 0 = DVB-T2 accumulator, 1 = dense generator
+  const uint64_t* enc_p;           // kind 1: k rows of words_m words (parity j of row i)
+  const int* enc_msg_cols;         // kind 1: k message columns
+  const int* enc_par_cols;         // kind 1: m parity columns
+  int enc_q;                       // kind 0: row groups (m / 360)
+  const int* enc_rg_ptr;           // kind 0: q + 1 offsets into enc_rg_ent
+  const int* enc_rg_ent;           // kind 0: info block b << 16 | rotation tau, per row group
+  int enc_rg_total;                // kind 0: entries of enc_rg_ent
+  int lay_dvb;                     // DVB-T2 layered kernels: slot bucket (0: not one of their codes)
+  int lay_runs;                    // most slots inside runs of one block in a row group
   // Structured variable edge lists (QC / DVB-T2 codes; sp_mode 0: none, use
   // sp_ci).  Edge lists per var group, {16 * (state index offset), slot |
   // wrap << 8}: the state of entry e for variable j of the group is at byte
@@ -87,17 +98,6 @@ struct DevCode {
                                    // the position offset, minus the var group's first variable
   int sp_nvd;                      // list entries of all groups
   int sp_ndesc;                    // entries of sp_desc
-  const int* csr_ptr;              // natural order H (m + 1)
-  const int* csr_idx;              // (nnz)
-  // encoder
-  int enc_kind;                    // 0 = DVB-T2 accumulator, 1 = dense generator
-  const uint64_t* enc_p;           // kind 1: k rows of words_m words (parity j of row i)
-  const int* enc_msg_cols;         // kind 1: k message columns
-  const int* enc_par_cols;         // kind 1: m parity columns
-  int enc_q;                       // kind 0: row groups (m / 360)
-  int enc_rg_total;                // kind 0: entries of enc_rg_ent
-  const int* enc_rg_ptr;           // kind 0: q + 1 offsets into enc_rg_ent
-  const int* enc_rg_ent;           // kind 0: info block b << 16 | rotation tau, per row group
 };
 
 uint64_t next_code_serial();
@@ -221,7 +221,6 @@ struct DecodeArgs {
   int smem_app_floats;             // APP kept in shared memory when n <= this
   int bitmap_words;                // 32-bit words of the hard-decision bitmap
   int lay_dbuf_off, lay_dbuf_floats;  // layered fused rows: shared-memory buffer of slots x checks
-  int lay_tab_off;                    // DVB-T2 layered kernels: row-group records and slot descriptors in smem
   int lay_stage_off, lay_stage_bytes; // layered, TMA-staged messages: two buffers of one row group's
                                       // messages, then two mbarriers (byte offset in dynamic smem)
   const float* alpha;              // NMS weights [nms_iters][nms_L]
@@ -235,8 +234,9 @@ struct DecodeArgs {
   // LLRs, the check states and the posteriors (frame state in the workspace)
   int sf_msg16;
   int sf_app_soff;
-  int sf_tab_off;                  // byte offset in shared memory of the structured tables (-1: not used)
   long long sf_llr_off, sf_st_off, sf_app_off;
+  int sf_tab_off;                  // byte offset in shared memory of the structured tables (-1: not used)
+  int lay_tab_off;                 // DVB-T2 layered kernels: row-group records and slot descriptors in smem
 };
 
 const void* flood_kernel_ptr(int algo, int msg16, int dcmax, int threads = 512);
