@@ -113,6 +113,7 @@ struct gf2c_decoder {
   StateFloodLayout sf_team{};
   int sf_teams[5] = {0, 0, 0, 0, 0};
   int team_threads = 0;
+  int64_t min_edges = 0;  // of the smallest code
   bool spa_flood = false;  // flooding sum-product of one DVB-T2 code (spa_flood.cu)
   long long sf_llr_off = 0, sf_st_off = 0, sf_app_off = 0;
   size_t smem = 0, work_bytes = 0;
@@ -569,7 +570,7 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     d->sf_app_off = L.app_off;
     d->work_stride = L.work_stride;
     d->smem = L.smem;
-    d->kernel = state_flood_kernel_ptr(sf_dc, L.all_smem);
+    d->kernel = state_flood_kernel_ptr(sf_dc, L);
     d->dcmax = sf_dc;
     threads = state_flood_threads();
     d->threads = threads;
@@ -686,13 +687,14 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
   // by two) stays with one.
   int64_t min_edges = INT64_MAX;
   for (auto* c : d->codes) min_edges = std::min(min_edges, (int64_t)c->h->row_idx.size());
+  d->min_edges = min_edges;
   if (d->spa_flood ||
       (d->state_flood && o.threads_per_block == 0 && o.blocks_per_sm == 0 && min_edges >= 24000)) {
     if (d->state_flood) {
       std::vector<const HostCode*> hc;
       for (auto* c : d->codes) hc.push_back(c->h.get());
       d->sf_team = state_flood_layout(hc, false);
-      d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, false);
+      d->sf_team_kernel = state_flood_kernel_ptr(d->dcmax, d->sf_team, true);
       d->team_threads = state_flood_threads();
     }
     GF2C_CUDA(allow_smem(d->sf_team_kernel, d->sf_team.smem));
@@ -751,13 +753,20 @@ static int team_of(const gf2c_decoder* d, int64_t frames) {
   if (!d->sf_team_kernel) return 0;
   static const float on_chip[5] = {1.0f, 0.74f, 0.54f, 0.42f, 0.35f};
   static const float in_memory[5] = {1.0f, 0.54f, 0.29f, 0.175f, 0.113f};
-  const float* t = d->sf_st_off == d->sf_app_off ? on_chip : in_memory;
+  const bool chip = d->sf_st_off == d->sf_app_off;
+  const float* t = chip ? on_chip : in_memory;
+  // The barriers' share of a team's time grows as the code shrinks against the
+  // normal DVB-T2 codes (220 K edges) that the second table is from: about 8000
+  // edges' worth (QC codes of 48 to 69 K edges, teams of two for 600 frames:
+  // 2.80, 3.55 and 3.78 ms, one CTA 2.55, 3.39 and 3.49 ms; for 200 frames teams
+  // of two stay 2 to 12 % ahead).
+  const float barriers = chip ? 0.0f : 8000.0f * std::max(0.0f, 1.0f / (float)d->min_edges - 1.0f / 220000.0f);
   int best = 0;
   float cost = 0.0f;
   for (int lg = 0; lg <= 4; lg++) {
     const int64_t slots = lg ? d->sf_teams[lg] : std::max(d->sf_slots[0], d->grid);
     if (slots <= 0) continue;
-    const float c = (float)((frames + slots - 1) / slots) * t[lg];
+    const float c = (float)((frames + slots - 1) / slots) * (t[lg] + (lg ? barriers : 0.0f));
     if (lg == 0 || c < cost) {
       best = lg;
       cost = c;

@@ -257,14 +257,16 @@ int state_flood_threads();
 // Memory layout of the check-state kernel for a set of codes: frame state in
 // shared memory (all_smem) or in the CTA's workspace slice, then the tables of
 // the structured passes in shared memory (tab_off -1: no structured pass).
+enum { kTables = 0, kStructured = 1, kBothPasses = 2 };
 struct StateFloodLayout {
   bool all_smem;
+  int passes;  // index tables only, structured only, or by each frame's code
   size_t smem;
   int app_soff, tab_off;
   long long llr_off, st_off, app_off, work_stride;
 };
 StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, bool on_chip = true);
-const void* state_flood_kernel_ptr(int dcmax, bool all_smem);
+const void* state_flood_kernel_ptr(int dcmax, const StateFloodLayout& L, bool team = false);
 // Flooding sum-product on DVB-T2 codes (spa_flood.cu), one kernel per bucket D of slots.
 int spa_flood_threads();
 StateFloodLayout spa_flood_layout(const std::vector<const HostCode*>& codes, int msg_bytes);

@@ -133,8 +133,7 @@ extern "C" int gf2c_decode_batch_noalloc(const gf2c_code* code, const float* llr
     smem = L.smem;
     sf_tab_off = L.tab_off;
     st_bytes = L.app_soff;
-    const bool all_smem = L.all_smem;
-    kern = state_flood_kernel_ptr(sf_dc, all_smem);
+    kern = state_flood_kernel_ptr(sf_dc, L);
     threads = state_flood_threads();
   } else {
     const int dcmax = decode_dcmax_bucket(h.max_dc);

@@ -461,13 +461,18 @@ __device__ __forceinline__ int sf_syndrome_pass(const Team team, const Post<ALL_
   return p;
 }
 
-template <int DCMAX, bool ALL_SMEM>
+// PASSES: StateFloodLayout::passes; TEAM: clusters of CTAs.  A kernel of its own
+// for each, since a CTA of 1024 threads has 64 registers per thread, and passes
+// that do not run or a team of one cost spills: 2000 frames of QC codes with the
+// state in the workspace, Z = 1024 without structured tables 10.6 -> 10.3 ms, 46 x
+// 68 blocks of Z = 384 9.79 -> 7.92 ms; 148 normal 1/2 frames 1.89 -> 1.68 ms.
+template <int DCMAX, bool ALL_SMEM, int PASSES, bool TEAM>
 __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const DecodeArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_frame[2];  // the frame (low, high word)
   __shared__ int s_vote[3];   // team votes: alternating iterations, final syndrome
   const DevCode& C = sf_code;
-  const Team team = Team::make(!ALL_SMEM);
+  const Team team = Team::make(TEAM);
   // thread index and count of the team
   const int tid = team.rank * (int)blockDim.x + (int)threadIdx.x, NT = team.size * (int)blockDim.x;
   const int lane = threadIdx.x & 31, ltid = threadIdx.x, LT = blockDim.x;
@@ -484,7 +489,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
       team.put(&s_frame[0], (int)(f & 0xffffffffll));
       team.put(&s_frame[1], (int)(f >> 32));
     }
-    if (ltid < 3) s_vote[ltid] = 0;
+    if (TEAM && ltid < 3) s_vote[ltid] = 0;
     team.sync();
     const long long f = (long long)s_frame[1] << 32 | (unsigned)s_frame[0];
     if (f < 0 || f >= a.frames) break;
@@ -536,7 +541,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
         }
       }
     }
-    const bool fast = a.sf_tab_off >= 0 && C.sp_mode != 0;
+    const bool fast = PASSES == kStructured || (PASSES == kBothPasses && a.sf_tab_off >= 0 && C.sp_mode != 0);
     FastTab T{};
     if (fast) {
       T = stage_tables(C, (int2*)(smem_raw + a.sf_tab_off), tab_code != cid);
@@ -550,18 +555,20 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
     int it = 0, converged = 0, synd = 1;
     for (;;) {
       const int nms_row = nms ? min(it, a.nms_iters - 1) * a.nms_L : 0;
-      int par = fast ? sf_check_fast<DCMAX>(team, T, st, P.p, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row,
-                                            a.nms_L == C.ncg)
-                     : sf_check_pass<DCMAX, ALL_SMEM>(team, st, P, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row,
-                                                      a.nms_L == C.ncg);
+      const bool per_layer = a.nms_L == C.ncg;
+      int par = 0;
+      if (PASSES != kTables && fast)
+        par = sf_check_fast<DCMAX>(team, T, st, P.p, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row, per_layer);
+      else if (PASSES != kStructured)
+        par = sf_check_pass<DCMAX, ALL_SMEM>(team, st, P, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row, per_layer);
       par = team.any(par, &s_vote[it & 1]);
-      if (ltid == 0) s_vote[(it + 1) & 1] = 0;  // used after the next barrier
+      if (TEAM && ltid == 0) s_vote[(it + 1) & 1] = 0;  // used after the next barrier
       if (it > 0 && a.early_stop && !par) {
         converged = 1;
         synd = 0;
         break;
       }
-      if (!fast) sf_var_pass<ALL_SMEM>(team, st, P, lu);
+      if (PASSES == kTables || (PASSES == kBothPasses && !fast)) sf_var_pass<ALL_SMEM>(team, st, P, lu);
       else if (C.sp_mode == 1) sf_var_fast<false>(team, T, st, P.p, lu);
       else sf_var_fast<true>(team, T, st, P.p, lu);
       team.sync();
@@ -601,31 +608,32 @@ int state_dcmax_bucket(int max_dc) {
   return -1;
 }
 
-template <bool ALL_SMEM>
+template <bool ALL_SMEM, int PASSES, bool TEAM>
 static const void* state_kernel(int dcmax) {
   switch (dcmax) {
-    case 7: return (const void*)bp_state_flood_kernel<7, ALL_SMEM>;
-    case 9: return (const void*)bp_state_flood_kernel<9, ALL_SMEM>;
-    case 10: return (const void*)bp_state_flood_kernel<10, ALL_SMEM>;
-    case 11: return (const void*)bp_state_flood_kernel<11, ALL_SMEM>;
-    case 13: return (const void*)bp_state_flood_kernel<13, ALL_SMEM>;
-    case 14: return (const void*)bp_state_flood_kernel<14, ALL_SMEM>;
-    case 18: return (const void*)bp_state_flood_kernel<18, ALL_SMEM>;
-    case 19: return (const void*)bp_state_flood_kernel<19, ALL_SMEM>;
-    case 22: return (const void*)bp_state_flood_kernel<22, ALL_SMEM>;
-    case 26: return (const void*)bp_state_flood_kernel<26, ALL_SMEM>;
-    case 32: return (const void*)bp_state_flood_kernel<32, ALL_SMEM>;
+    case 7: return (const void*)bp_state_flood_kernel<7, ALL_SMEM, PASSES, TEAM>;
+    case 9: return (const void*)bp_state_flood_kernel<9, ALL_SMEM, PASSES, TEAM>;
+    case 10: return (const void*)bp_state_flood_kernel<10, ALL_SMEM, PASSES, TEAM>;
+    case 11: return (const void*)bp_state_flood_kernel<11, ALL_SMEM, PASSES, TEAM>;
+    case 13: return (const void*)bp_state_flood_kernel<13, ALL_SMEM, PASSES, TEAM>;
+    case 14: return (const void*)bp_state_flood_kernel<14, ALL_SMEM, PASSES, TEAM>;
+    case 18: return (const void*)bp_state_flood_kernel<18, ALL_SMEM, PASSES, TEAM>;
+    case 19: return (const void*)bp_state_flood_kernel<19, ALL_SMEM, PASSES, TEAM>;
+    case 22: return (const void*)bp_state_flood_kernel<22, ALL_SMEM, PASSES, TEAM>;
+    case 26: return (const void*)bp_state_flood_kernel<26, ALL_SMEM, PASSES, TEAM>;
+    case 32: return (const void*)bp_state_flood_kernel<32, ALL_SMEM, PASSES, TEAM>;
   }
   return nullptr;
 }
 
 StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, bool on_chip) {
   size_t max_m = 0, max_n = 0, tab = 0;
-  bool any_perm = false, any_fast = false;
+  bool any_perm = false, any_fast = false, all_fast = true;
   for (const HostCode* h : codes) {
     max_m = std::max(max_m, (size_t)h->m);
     max_n = std::max(max_n, (size_t)h->n);
     any_perm = any_perm || !h->sp_u2v.empty();
+    all_fast = all_fast && h->sp_mode != 0;
     if (h->sp_mode) {
       any_fast = true;
       tab = std::max(tab, 8 * (h->sp_desc.size() + h->cg.size() + h->sp_vh.size() + h->sp_vd.size()));
@@ -645,6 +653,9 @@ StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, b
   if (!fits) app_bytes = max_n * 4;
   L.app_soff = (int)st_bytes;
   L.tab_off = fits ? (int)state : -1;
+  // (In the workspace the kernel with both kinds of passes serves the structured
+  // ones alone too: 148 normal 3/5 frames 1.82 ms, 2.08 ms without the others.)
+  L.passes = !fits ? kTables : all_fast && L.all_smem ? kStructured : kBothPasses;
   L.smem = fits ? state + tab : (L.all_smem ? st_bytes + max_n * 4 : 0);
   auto al = [](size_t x) { return (long long)((x + 255) / 256 * 256); };
   long long off = 0;
@@ -658,8 +669,15 @@ StateFloodLayout state_flood_layout(const std::vector<const HostCode*>& codes, b
   return L;
 }
 
-const void* state_flood_kernel_ptr(int dcmax, bool all_smem) {
-  return all_smem ? state_kernel<true>(dcmax) : state_kernel<false>(dcmax);
+const void* state_flood_kernel_ptr(int dcmax, const StateFloodLayout& L, bool team) {
+  if (team)
+    return L.passes == kTables ? state_kernel<false, kTables, true>(dcmax) : state_kernel<false, kBothPasses, true>(dcmax);
+  if (!L.all_smem)
+    return L.passes == kTables ? state_kernel<false, kTables, false>(dcmax)
+                               : state_kernel<false, kBothPasses, false>(dcmax);
+  return L.passes == kTables       ? state_kernel<true, kTables, false>(dcmax)
+         : L.passes == kStructured ? state_kernel<true, kStructured, false>(dcmax)
+                                   : state_kernel<true, kBothPasses, false>(dcmax);
 }
 
 }  // namespace gf2c
