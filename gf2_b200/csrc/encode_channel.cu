@@ -79,12 +79,16 @@ __device__ __forceinline__ void dvbt2_build_blocks(const uint32_t* u, int pitch,
 }
 
 // S[13 a + w] = word w (t = 32 w + bit) of the info syndrome of row group a,
-// W words per task (13: a warp reads one word of 32 row groups).
+// W words per task (13: a warp reads one word of 32 row groups).  With one or two
+// words per task the tasks of a row group are neighbours, so that a warp reads few
+// table entries and runs of words (the encoder in the channel kernel, 3000 normal
+// 3/5 frames: 86 us, 99 us with a warp across 32 row groups).
 template <int W, int G>
 __device__ __forceinline__ void dvbt2_row_syndromes(const int* __restrict__ rg_ptr, const uint32_t* ent,
                                                     const Words<G>* U2, int q, Words<G>* S) {
   for (int idx = threadIdx.x; idx < (12 / W) * q; idx += blockDim.x) {
-    const int part = idx / q, a = idx - part * q;
+    constexpr int parts = 12 / W;
+    const int a = W <= 2 ? idx / parts : idx % q, part = W <= 2 ? idx - a * parts : idx / q;
     Words<G> acc[W];
 #pragma unroll
     for (int i = 0; i < W; i++)
@@ -455,6 +459,33 @@ __global__ void __launch_bounds__(256) syndrome_kernel(const DevCode* __restrict
   }
 }
 
+// LLRs of one frame with codeword bits c.  Not inlined: the loop is bound by FP64
+// arithmetic and wants the registers that the encoder in front of it would hold
+// (3000 normal 3/5 frames: 1.51 ms inlined, 1.41 ms).
+__device__ __noinline__ void channel_llrs(const uint32_t* c, int n, uint32_t fr, uint2 key, double s2, float* lo) {
+  const double sigma = __dsqrt_rn(s2);
+  for (int pair = threadIdx.x; 2 * pair < n; pair += blockDim.x) {
+    const uint4 r = philox4x32_10(make_uint4((uint32_t)pair, fr, 2u, 0u), key);
+    const unsigned long long a = (((unsigned long long)r.x << 32) | r.y) >> 11;
+    const unsigned long long b = (((unsigned long long)r.z << 32) | r.w) >> 11;
+    const double u1 = __dmul_rn((double)(a + 1ull), 1.1102230246251565404e-16);
+    const double u2 = __dmul_rn((double)b, 1.1102230246251565404e-16);
+    const double rad = __dsqrt_rn(__dmul_rn(-2.0, log_d(u1)));
+    double sn, cs;
+    sincos_2pi_d(u2, &sn, &cs);
+    const double z[2] = {__dmul_rn(rad, cs), __dmul_rn(rad, sn)};
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int i = 2 * pair + h;
+      if (i < n) {
+        const double sym = getbit(c, i) ? -1.0 : 1.0;
+        const double y = __dadd_rn(sym, __dmul_rn(sigma, z[h]));
+        lo[i] = __double2float_rn(__ddiv_rn(__dmul_rn(2.0, y), s2));
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kEncThreads) channel_kernel(const DevCode* __restrict__ Cp, uint2 key,
                                                               unsigned long long frame0, long long frames,
                                                               const double* __restrict__ sigma2,
@@ -494,31 +525,7 @@ __global__ void __launch_bounds__(kEncThreads) channel_kernel(const DevCode* __r
       uint32_t* co = (uint32_t*)(cwo + f * (long long)C.words_n);
       for (int w = threadIdx.x; w < 2 * C.words_n; w += blockDim.x) co[w] = w < wn ? c[w] : 0u;
     }
-    if (llr) {
-      const double s2 = sigma2[f];
-      const double sigma = __dsqrt_rn(s2);
-      float* lo = llr + f * (long long)C.n;
-      for (int pair = threadIdx.x; 2 * pair < C.n; pair += blockDim.x) {
-        const uint4 r = philox4x32_10(make_uint4((uint32_t)pair, fr, 2u, 0u), key);
-        const unsigned long long a = (((unsigned long long)r.x << 32) | r.y) >> 11;
-        const unsigned long long b = (((unsigned long long)r.z << 32) | r.w) >> 11;
-        const double u1 = __dmul_rn((double)(a + 1ull), 1.1102230246251565404e-16);
-        const double u2 = __dmul_rn((double)b, 1.1102230246251565404e-16);
-        const double rad = __dsqrt_rn(__dmul_rn(-2.0, log_d(u1)));
-        double sn, cs;
-        sincos_2pi_d(u2, &sn, &cs);
-        const double z[2] = {__dmul_rn(rad, cs), __dmul_rn(rad, sn)};
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int i = 2 * pair + h;
-          if (i < C.n) {
-            const double sym = getbit(c, i) ? -1.0 : 1.0;
-            const double y = __dadd_rn(sym, __dmul_rn(sigma, z[h]));
-            lo[i] = __double2float_rn(__ddiv_rn(__dmul_rn(2.0, y), s2));
-          }
-        }
-      }
-    }
+    if (llr) channel_llrs(c, C.n, fr, key, sigma2[f], llr + f * (long long)C.n);
     __syncthreads();
   }
 }
