@@ -1010,8 +1010,17 @@ int gf2c_bch_create_dvbt2(int32_t frame_size, int32_t rate, gf2c_bch** out) {
   auto mul = [&](uint32_t a, uint32_t c) -> uint32_t {
     return (a && c) ? b->h_exp[b->h_log[a] + b->h_log[c]] : 0u;
   };
+  // z^2 + z is linear over GF(2): one bit of z at a time (Gray code)
   b->h_half.assign(q, 0);
-  for (uint32_t z = 2; z < (uint32_t)q; z++) b->h_half[mul(z, z) ^ z] = (uint16_t)z;
+  uint16_t image[16];
+  for (int e = 0; e < d.m; e++) image[e] = (uint16_t)(mul(1u << e, 1u << e) ^ (1u << e));
+  for (uint32_t i = 1, z = 0, c = 0; i < (uint32_t)q; i++) {
+    const int e = __builtin_ctz(i);
+    z ^= 1u << e;
+    c ^= image[e];
+    b->h_half[c] = (uint16_t)(z | 1u);
+  }
+  b->h_half[0] = 0;  // z = 0 and 1
   // generator g = g_1 ... g_t (binary)
   std::vector<uint8_t> g{1};
   for (int i = 0; i < d.t; i++) {
@@ -1039,11 +1048,10 @@ int gf2c_bch_create_dvbt2(int32_t frame_size, int32_t rate, gf2c_bch** out) {
     for (int p = 0; p < 8; p++) {
       uint32_t unit[8];
       for (int e = 0; e < 8; e++) unit[e] = apow(-j * (8 * p + e));
-      for (int v = 0; v < 256; v++) {
-        uint64_t acc = 0;
-        for (int e = 0; e < 8; e++)
-          if ((v >> e) & 1) acc ^= unit[e];
-        b->h_quad[((size_t)(s / 4) * 8 + p) * 256 + v] |= acc << (16 * (s % 4));
+      uint64_t sum[256] = {0};  // each from the one without its lowest bit
+      for (int v = 1; v < 256; v++) {
+        sum[v] = sum[v & (v - 1)] ^ unit[__builtin_ctz(v)];
+        b->h_quad[((size_t)(s / 4) * 8 + p) * 256 + v] |= sum[v] << (16 * (s % 4));
       }
     }
     const uint32_t gamma = apow(-j * 2048);
