@@ -28,16 +28,11 @@ int cuda_error(cudaError_t e, const char* what) {
 
 cudaError_t allow_smem(const void* kernel, size_t bytes) {
   static std::mutex mu;
-  static std::map<std::pair<int, const void*>, size_t> limits;  // per device and kernel
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
-  size_t& limit = limits[{dev, kernel}];
-  if (bytes <= limit) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) limit = bytes;
-  return e;
+  cudaFuncAttributes at;  // read from the context each time (0.3 us), which may be a new one
+  const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess || bytes <= (size_t)at.maxDynamicSharedSizeBytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // Device buffer that only grows.
