@@ -107,6 +107,8 @@ struct gf2c_decoder {
   const void* sf_team_kernel = nullptr;
   StateFloodLayout sf_team{};
   int sf_teams[5] = {0, 0, 0, 0, 0};
+  bool teams_known = false;  // sf_teams asked for (by the first batch that may want a team)
+  int team_ctas = 0;         // CTAs of the team kernel in flight: the workspace holds team_ctas / 2 teams
   int team_threads = 0;
   int64_t min_edges = 0;  // of the smallest code
   bool spa_flood = false;  // flooding sum-product of one DVB-T2 code (spa_flood.cu)
@@ -694,17 +696,10 @@ int gf2c_decoder_create_multi(const gf2c_code* const* codes, int32_t ncodes, con
     }
     GF2C_CUDA(allow_smem(d->sf_team_kernel, d->sf_team.smem));
     GF2C_CUDA(cudaFuncSetAttribute(d->sf_team_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    for (int lg = 1; lg <= 4; lg++) {
-      cudaLaunchAttribute at;
-      cudaLaunchConfig_t cfg = team_config(d.get(), 1 << lg, 1, nullptr, &at);
-      int nc = 0;
-      if (cudaOccupancyMaxActiveClusters(&nc, d->sf_team_kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        nc = 0;
-      }
-      d->sf_teams[lg] = nc;
-      work_bytes = std::max(work_bytes, (size_t)d->sf_team.work_stride * nc);
-    }
+    int b = 0;
+    GF2C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, d->sf_team_kernel, d->team_threads, d->sf_team.smem));
+    d->team_ctas = sms * b;
+    work_bytes = std::max(work_bytes, (size_t)d->sf_team.work_stride * (d->team_ctas / 2));
   }
   if ((rc = d->work.ensure(work_bytes))) return rc;
   d->work_bytes = work_bytes;
@@ -730,6 +725,23 @@ int gf2c_decoder_last_launches(const gf2c_decoder* dec, int32_t* launches) {
   return GF2C_OK;
 }
 
+// Teams in flight per size: asked for once, by the first batch that may want one
+// (four queries, which a decoder of large batches need not wait for).
+static void find_teams(gf2c_decoder* d) {
+  if (d->teams_known) return;
+  d->teams_known = true;
+  for (int lg = 1; lg <= 4; lg++) {
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = team_config(d, 1 << lg, 1, nullptr, &at);
+    int nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, d->sf_team_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      nc = 0;
+    }
+    d->sf_teams[lg] = std::min(nc, d->team_ctas >> lg);
+  }
+}
+
 // CTAs per frame (log2) of a flooding decode of `frames` frames.  Min-sum: the
 // team with the shortest estimate, waves times the time of a frame (relative to
 // one CTA, measured on short 1/2 with its state on chip and on normal 3/5:
@@ -738,14 +750,16 @@ int gf2c_decoder_last_launches(const gf2c_decoder* dec, int32_t* launches) {
 // frames: 0.87 ms by teams of 4, 0.74 ms by teams of 8 in three waves), and two
 // CTAs per frame beat one for every batch (1000 frames 8.4 ms both, 256 frames
 // 2.69 against 3.27 ms, 2.78 ms by teams of 4).
-static int team_of(const gf2c_decoder* d, int64_t frames) {
+static int team_of(gf2c_decoder* d, int64_t frames) {
+  // No team for many waves: twice a team of two's time is 1.08 times one CTA's.
+  if (!d->sf_team_kernel || (!d->spa_flood && frames >= 16 * (int64_t)d->grid)) return 0;
+  find_teams(d);
   if (d->spa_flood) {
     if (frames <= d->sf_teams[4]) return 4;
     if (frames <= 3 * (int64_t)d->sf_teams[3]) return 3;
     if (frames <= 3 * (int64_t)d->sf_teams[2]) return 2;
     return d->sf_teams[1] > 0 ? 1 : 0;
   }
-  if (!d->sf_team_kernel) return 0;
   static const float on_chip[5] = {1.0f, 0.74f, 0.54f, 0.42f, 0.35f};
   static const float in_memory[5] = {1.0f, 0.54f, 0.29f, 0.175f, 0.113f};
   const bool chip = d->sf_st_off == d->sf_app_off;
