@@ -35,6 +35,55 @@ cudaError_t allow_smem(const void* kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Pinned host buffers of small host-memory batches, in two sizes.  Making one takes
+// 1 to 2.6 ms and freeing it 0.4 ms, more than a decode, so those of destroyed
+// decoders wait here for the next one: at most kKeep of each size, the others are
+// freed.
+class PinnedPool {
+ public:
+  static constexpr size_t kBytes[2] = {1 << 17, 1 << 20};
+  // A buffer of size class c; where none waits, a new one or (`make` false) null.
+  void* take(int c, bool make) {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      while (kept_[c] > 0) {
+        void* p = free_[c][--kept_[c]];
+        cudaPointerAttributes at;  // a device reset in between takes the memory away
+        if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost) return p;
+        cudaGetLastError();
+      }
+    }
+    void* p = nullptr;
+    if (make && cudaMallocHost(&p, kBytes[c]) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return p;
+  }
+  void give(int c, void* p) {
+    if (!p) return;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      if (kept_[c] < kKeep) {
+        free_[c][kept_[c]++] = p;
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr int kKeep = 4;
+  std::mutex mu_;
+  void* free_[2][kKeep] = {};
+  int kept_[2] = {0, 0};
+};
+constexpr size_t PinnedPool::kBytes[2];
+static PinnedPool& pinned_pool() {
+  static PinnedPool* pool = new PinnedPool;  // never destroyed: decoders may outlive static objects
+  return *pool;
+}
+
 // Device buffer that only grows.
 struct DevBuf {
   void* p = nullptr;
@@ -119,9 +168,10 @@ struct gf2c_decoder {
   int nms_iters = 0, nms_L = 0;
   // staging for host-memory calls
   DevBuf s_llr, s_msg, s_it, s_cv, s_so, s_bel, s_off1, s_off2, s_cid, s_mit;
-  // pinned buffer of small host-memory batches (at most kSmallHost bytes)
+  // pinned buffer of small host-memory batches (PinnedPool, size class; -1: none)
   void* h_small = nullptr;
-  size_t h_small_bytes = 0;
+  int h_small_class = -1;
+  int small_calls = 0;
   int last_launches = 0;
   std::map<GraphKey, cudaGraphExec_t> graphs;
   cudaStream_t gstream = nullptr;
@@ -145,7 +195,7 @@ struct gf2c_decoder {
   DevBuf fb_list, fb_count;
   ~gf2c_decoder() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
-    if (h_small) cudaFreeHost(h_small);
+    if (h_small) pinned_pool().give(h_small_class, h_small);
     if (gstream) {
       cudaStreamSynchronize(gstream);
       cudaStreamDestroy(gstream);
@@ -935,22 +985,55 @@ static bool pipeline_ready(gf2c_decoder* d) {
   return true;
 }
 
-static constexpr size_t kSmallHost = 1 << 20;
+static constexpr size_t kSmallHost = PinnedPool::kBytes[1];
 
 // The decoder's pinned buffer with room for `bytes` (at most kSmallHost); false
-// where it cannot be had.
+// where it has none.  A decoder whose first calls find none waiting goes without
+// for kPatience calls: a new one costs as much as it saves in some thirty calls (40
+// us each), and a decoder made for one call should not pay for it.
 static bool small_host(gf2c_decoder* d, size_t bytes) {
-  if (bytes <= d->h_small_bytes) return true;
-  const size_t want = bytes <= kSmallHost / 8 ? kSmallHost / 8 : kSmallHost;
-  void* p = nullptr;
-  if (cudaMallocHost(&p, want) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (d->h_small) cudaFreeHost(d->h_small);
+  static constexpr int kPatience = 8;
+  const int c = bytes <= PinnedPool::kBytes[0] ? 0 : 1;
+  if (c <= d->h_small_class) return true;
+  void* p = pinned_pool().take(c, d->small_calls >= kPatience);
+  if (d->small_calls < kPatience) d->small_calls++;
+  if (!p) return false;
+  if (d->h_small) pinned_pool().give(d->h_small_class, d->h_small);
   d->h_small = p;
-  d->h_small_bytes = want;
+  d->h_small_class = c;
   return true;
+}
+
+// A small host-memory batch through the pinned buffer: the copies' own latency is a
+// third of such a call, so the LLRs go through pinned memory and the outputs come
+// back in one copy next to the status word (one short 1/2 frame: 187 -> 142 us a
+// call).  On an error the stream may still be copying from the buffer.
+static int small_batch(gf2c_decoder* dec, DecodeArgs a, const float* llr, int64_t frames, size_t bl, size_t bm,
+                       uint64_t* msg_bits, int32_t* iterations, uint8_t* converged, uint8_t* syndrome_ok,
+                       cudaStream_t st) {
+  const size_t bout = bm + (size_t)frames * 6;
+  char* hb = (char*)dec->h_small;
+  int rc, extra = 0;
+  if ((rc = dec->s_llr.ensure(bl)) || (rc = dec->s_msg.ensure(bout))) return rc;
+  char* db = (char*)dec->s_msg.p;
+  std::memcpy(hb, llr, bl);
+  GF2C_CUDA(cudaMemcpyAsync(dec->s_llr.p, hb, bl, cudaMemcpyHostToDevice, st));
+  a.llr = (const float*)dec->s_llr.p;
+  a.msg = (uint64_t*)db;
+  a.iters = (int32_t*)(db + bm);
+  a.conv = (uint8_t*)(db + bm + (size_t)frames * 4);
+  a.synd_ok = a.conv + frames;
+  if ((rc = key_order(dec, a, frames, st, 0, extra))) return rc;
+  if ((rc = launch_decoder(dec, a, frames, st))) return rc;
+  dec->last_launches += extra;
+  char* ho = hb + bl;
+  GF2C_CUDA(cudaMemcpyAsync(ho, db, bout, cudaMemcpyDeviceToHost, st));
+  if ((rc = check_status(dec, st, ho + bout))) return rc;
+  if (msg_bits) std::memcpy(msg_bits, ho, bm);
+  if (iterations) std::memcpy(iterations, ho + bm, (size_t)frames * 4);
+  if (converged) std::memcpy(converged, ho + bm + (size_t)frames * 4, (size_t)frames);
+  if (syndrome_ok) std::memcpy(syndrome_ok, ho + bm + (size_t)frames * 5, (size_t)frames);
+  return GF2C_OK;
 }
 
 int gf2c_decode_batch(gf2c_decoder* dec, const float* llr, int64_t frames, int32_t max_iter, uint64_t* msg_bits,
@@ -979,34 +1062,12 @@ int gf2c_decode_batch(gf2c_decoder* dec, const float* llr, int64_t frames, int32
   }
   const int wk = (int)((h.k + 63) / 64);
   size_t bl = (size_t)frames * h.n * 4, bm = (size_t)frames * wk * 8;
-  // Small batches (a frame or a few as they arrive): the copies' own latency is
-  // a third of the call, so the LLRs go through a pinned buffer and the outputs
-  // come back in one copy next to the status word (one short 1/2 frame: 187 ->
-  // 142 us a call).
-  const size_t bout = bm + (size_t)frames * 6;
-  if (!beliefs && bl + bout + 16 <= kSmallHost && small_host(dec, bl + bout + 16)) {
-    char* hb = (char*)dec->h_small;
-    if ((rc = dec->s_llr.ensure(bl)) || (rc = dec->s_msg.ensure(bout))) return rc;
-    char* db = (char*)dec->s_msg.p;
-    std::memcpy(hb, llr, bl);
-    GF2C_CUDA(cudaMemcpyAsync(dec->s_llr.p, hb, bl, cudaMemcpyHostToDevice, st));
-    a.llr = (const float*)dec->s_llr.p;
-    a.msg = (uint64_t*)db;
-    a.iters = (int32_t*)(db + bm);
-    a.conv = (uint8_t*)(db + bm + (size_t)frames * 4);
-    a.synd_ok = a.conv + frames;
-    int extra = 0;
-    if ((rc = key_order(dec, a, frames, st, 0, extra))) return rc;
-    if ((rc = launch_decoder(dec, a, frames, st))) return rc;
-    dec->last_launches += extra;
-    char* ho = hb + bl;
-    GF2C_CUDA(cudaMemcpyAsync(ho, db, bout, cudaMemcpyDeviceToHost, st));
-    if ((rc = check_status(dec, st, ho + bout))) return rc;
-    if (msg_bits) std::memcpy(msg_bits, ho, bm);
-    if (iterations) std::memcpy(iterations, ho + bm, (size_t)frames * 4);
-    if (converged) std::memcpy(converged, ho + bm + (size_t)frames * 4, (size_t)frames);
-    if (syndrome_ok) std::memcpy(syndrome_ok, ho + bm + (size_t)frames * 5, (size_t)frames);
-    return GF2C_OK;
+  // a frame or a few as they arrive
+  const size_t small = bl + bm + (size_t)frames * 6 + 16;
+  if (!beliefs && small <= kSmallHost && small_host(dec, small)) {
+    rc = small_batch(dec, a, llr, frames, bl, bm, msg_bits, iterations, converged, syndrome_ok, st);
+    if (rc) cudaStreamSynchronize(st);
+    return rc;
   }
   if ((rc = dec->s_llr.ensure(bl)) || (rc = dec->s_msg.ensure(bm)) || (rc = dec->s_it.ensure(frames * 4)) ||
       (rc = dec->s_cv.ensure(frames)) || (rc = dec->s_so.ensure(frames)))

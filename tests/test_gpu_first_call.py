@@ -23,3 +23,35 @@ def test_first_call_under_capture(gpu, algo, frames):
     graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(out[k], ref[k]) for k in ref)
+
+
+def test_small_host_batches_with_and_without_a_pinned_buffer(gpu):
+    """More calls than a new decoder waits for its buffer, sizes of both classes in
+    turn, decoders that come and go in several threads: always the device call's
+    results."""
+    import threading
+
+    import numpy as np
+    import torch
+    code = g.LdpcCode.dvb_t2_short(0)
+    rng = np.random.default_rng(1)
+    xs = [rng.normal(2.0, 2.0, (f, code.n())).astype(np.float32) for f in (1, 3, 14)]
+    dev = g.LdpcDecoder(code)
+    ref = [{k: v.cpu().numpy() for k, v in dev.decode_tensors(torch.from_numpy(x).to(gpu), 4).items()} for x in xs]
+    wrong = []
+
+    def work(turn):
+        for life in range(3):
+            dec = g.LdpcDecoder(code)
+            for call in range(12):
+                i = (turn + life + call // 2) % len(xs)
+                r = dec.decode_arrays(xs[i], 4)
+                if not all((np.asarray(r[k]).astype(np.int64) == ref[i][k].astype(np.int64)).all() for k in ref[i]):
+                    wrong.append((turn, life, call))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
