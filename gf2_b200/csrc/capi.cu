@@ -135,10 +135,11 @@ struct gf2c_decoder {
   const void* lay_many_kernel = nullptr;
   int lay_many_threads = 0, lay_many_grid = 0, lay_few_grid = 0;
   // Frames in flight of the plain launch shape: what a chunk of the host-memory
-  // pipelines holds at least.  The larger grids of the shapes above and below
-  // would make the chunks too few to overlap copies and decoding (learned decoder
-  // with fallback, 1500 normal 2/3 frames from pinned memory: 10.3 ms in chunks of
-  // 296 frames and more, 15.3 ms in chunks of 592).
+  // call with fallback holds at least.  The larger grids of the shapes above and
+  // below would make its chunks too few to overlap copies and decoding (learned
+  // decoder, 1500 normal 2/3 frames from pinned memory: 10.3 ms in chunks of 296
+  // frames and more, 15.3 ms in chunks of 592).  Without a fallback the copies are
+  // the longer part, and larger chunks are ahead (4096 frames 38.3 and 40.1 ms).
   int wave = 0;
   bool state_flood = false;  // check-state flooding min-sum kernel (state_flood.cu)
   int sf_app_soff = 0, sf_tab_off = -1;
@@ -1082,15 +1083,15 @@ int gf2c_decode_batch(gf2c_decoder* dec, const float* llr, int64_t frames, int32
   // frame queue).  Only the last chunk is decoded hardest frames first: the
   // ordering kernels of the others would wait for those SMs, which the next
   // chunk's decode fills anyway.
-  const int64_t chunk = std::max<int64_t>(dec->wave, (frames + 7) / 8);
+  const int64_t chunk = std::max<int64_t>(dec->grid, (frames + 7) / 8);
   if (frames >= 2 * chunk && bl >= ((size_t)64 << 20) && pipeline_ready(dec)) {
     GF2C_CUDA(cudaEventRecord(dec->pev_fork, st));
     GF2C_CUDA(cudaStreamWaitEvent(dec->pstream, dec->pev_fork, 0));
     GF2C_CUDA(cudaStreamWaitEvent(dec->cstream, dec->pev_fork, 0));
     int chunks = 0, launches = 0;
-    const int64_t csz = even_chunk(frames, dec->wave);
+    const int64_t csz = even_chunk(frames, dec->grid);
     for (int64_t f0 = 0, nf = 0; f0 < frames; f0 += nf, chunks++) {
-      nf = chunk_frames(csz, frames - f0, dec->wave);
+      nf = chunk_frames(csz, frames - f0, dec->grid);
       const int slot = chunks & 1;
       cudaStream_t s = slot ? dec->pstream : st;
       const size_t ln = (size_t)nf * h.n * 4, lo = (size_t)f0 * h.n * 4;
@@ -1454,7 +1455,7 @@ int gf2c_decode_mixed(gf2c_decoder* dec, const float* llr, const int64_t* llr_of
   // gf2c_decode_batch).  The frame order of a chunk (code by code, longest
   // codes first, then by frame index, the ordering kernel's rule) is made on
   // the host; the persistent kernel takes the chunk's frames from it.
-  const int64_t wave = dec->wave;
+  const int64_t wave = dec->grid;
   if (ordered && frames >= 3 * wave && (size_t)llr_total * 4 >= ((size_t)64 << 20) && pipeline_ready(dec) &&
       dec->s_cnt.ensure(64 * 8) == GF2C_OK) {
     std::vector<int64_t> mem((size_t)frames), ord((size_t)frames);
