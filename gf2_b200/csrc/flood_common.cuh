@@ -31,10 +31,6 @@ struct Team {
   }
   // Stores v to the shared variable at p in every CTA of the team.
   __device__ __forceinline__ void put(int* p, int v) const {
-    if (size == 1) {
-      *p = v;
-      return;
-    }
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
     for (int r = 0; r < size; r++)
       asm volatile("{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %0, %1;\n st.shared::cluster.u32 [ra], %2;\n}" ::"r"(a),

@@ -486,8 +486,13 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
       const long long q = (long long)atomicAdd(a.queue, 1ull);
       const long long nq = a.frames_dev ? *a.frames_dev : a.frames;  // queue entries
       const long long f = (q < nq) ? (a.order != nullptr ? a.order[q] : q) : -1;
-      team.put(&s_frame[0], (int)(f & 0xffffffffll));
-      team.put(&s_frame[1], (int)(f >> 32));
+      if (TEAM) {
+        team.put(&s_frame[0], (int)(f & 0xffffffffll));
+        team.put(&s_frame[1], (int)(f >> 32));
+      } else {
+        s_frame[0] = (int)(f & 0xffffffffll);
+        s_frame[1] = (int)(f >> 32);
+      }
     }
     if (TEAM && ltid < 3) s_vote[ltid] = 0;
     team.sync();
@@ -555,12 +560,11 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
     int it = 0, converged = 0, synd = 1;
     for (;;) {
       const int nms_row = nms ? min(it, a.nms_iters - 1) * a.nms_L : 0;
-      const bool per_layer = a.nms_L == C.ncg;
-      int par = 0;
-      if (PASSES != kTables && fast)
-        par = sf_check_fast<DCMAX>(team, T, st, P.p, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row, per_layer);
-      else if (PASSES != kStructured)
-        par = sf_check_pass<DCMAX, ALL_SMEM>(team, st, P, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row, per_layer);
+      int par = PASSES != kTables && fast
+                    ? sf_check_fast<DCMAX>(team, T, st, P.p, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row,
+                                           a.nms_L == C.ncg)
+                    : sf_check_pass<DCMAX, ALL_SMEM>(team, st, P, it == 0, nms, a.sf_msg16 != 0, a.alpha, a.beta, nms_row,
+                                                     a.nms_L == C.ncg);
       par = team.any(par, &s_vote[it & 1]);
       if (TEAM && ltid == 0) s_vote[(it + 1) & 1] = 0;  // used after the next barrier
       if (it > 0 && a.early_stop && !par) {
@@ -568,7 +572,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) bp_state_flood_kernel(const 
         synd = 0;
         break;
       }
-      if (PASSES == kTables || (PASSES == kBothPasses && !fast)) sf_var_pass<ALL_SMEM>(team, st, P, lu);
+      if (PASSES == kTables || !fast) sf_var_pass<ALL_SMEM>(team, st, P, lu);
       else if (C.sp_mode == 1) sf_var_fast<false>(team, T, st, P.p, lu);
       else sf_var_fast<true>(team, T, st, P.p, lu);
       team.sync();
