@@ -798,9 +798,14 @@ static void find_teams(gf2c_decoder* d) {
 // one CTA, measured on short 1/2 with its state on chip and on normal 3/5:
 // sf_teams).  Sum-product: frames differ more in iterations than in anything
 // else, so a few waves of larger teams beat one of smaller ones (37 short 1/2
-// frames: 0.87 ms by teams of 4, 0.74 ms by teams of 8 in three waves), and two
-// CTAs per frame beat one for every batch (1000 frames 8.4 ms both, 256 frames
-// 2.69 against 3.27 ms, 2.78 ms by teams of 4).
+// frames: 0.87 ms by teams of 4, 0.74 ms by teams of 8 in three waves).  Larger
+// batches (600 frames at the waterfall, 15 iterations, exact with FP32 messages and
+// SFU with FP16): normal codes by two CTAs per frame (rate 3/5 14.3 and 8.6 ms, 15.5
+// and 10.3 ms by one; 3/4 12.1 and 8.5 ms, 15.3 and 9.8 ms by one).  Short codes of up
+// to 11 slots, two of whose CTAs fit an SM, by two as well (3/5: 3.00 and 1.87 ms,
+// 3.14 and 1.81 ms by one; one is up to 1.2 times as fast around 300
+// frames and as slow at 256).  Short codes of more slots, one CTA per SM, by one
+// from a whole wave on (3/4: 3.06 and 1.52 ms, 3.85 and 2.31 ms by two).
 static int team_of(gf2c_decoder* d, int64_t frames) {
   // No team for many waves: twice a team of two's time is 1.08 times one CTA's.
   if (!d->sf_team_kernel || (!d->spa_flood && frames >= 16 * (int64_t)d->grid)) return 0;
@@ -809,6 +814,7 @@ static int team_of(gf2c_decoder* d, int64_t frames) {
     if (frames <= d->sf_teams[4]) return 4;
     if (frames <= 3 * (int64_t)d->sf_teams[3]) return 3;
     if (frames <= 3 * (int64_t)d->sf_teams[2]) return 2;
+    if (d->max_n <= 16200 && d->max_dc > 11 && frames >= d->grid) return 0;
     return d->sf_teams[1] > 0 ? 1 : 0;
   }
   static const float on_chip[5] = {1.0f, 0.74f, 0.54f, 0.42f, 0.35f};
