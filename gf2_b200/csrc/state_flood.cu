@@ -34,8 +34,9 @@
 // every slot of every row group reads a contiguous, rotated run of Z
 // posteriors and every variable group reads contiguous check states.
 //
-// Batches of fewer frames than SMs: a cluster of 2 to 16 CTAs takes a frame
-// (struct Team), with the frame state in the workspace.
+// Batches that leave SMs idle, or would in their last wave: a cluster of 2 to 16
+// CTAs takes a frame (struct Team), with the frame state in the workspace.  Which
+// size, if any, is estimated per batch (team_of in capi.cu).
 //
 // Placement.  The check states (m x 16 B) and the posteriors (n x 4 B) live in
 // shared memory when they fit together (DVB-T2 short frames, ALL_SMEM);
